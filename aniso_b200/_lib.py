@@ -50,6 +50,9 @@ EXPORTS = [
     "aniso_b200_sort_projection_noalloc",
     "aniso_b200_scene_load_ply",
     "aniso_b200_adam_step",
+    "aniso_b200_loss_work_floats",
+    "aniso_b200_loss_forward",
+    "aniso_b200_loss_backward",
     "aniso_b200_colmap_load",
 ]
 
@@ -116,6 +119,9 @@ def _load():
         "aniso_b200_scene_destroy": [P],
         "aniso_b200_scene_load_ply": [ctypes.c_char_p, ctypes.POINTER(P)],
         "aniso_b200_adam_step": [ctypes.POINTER(AdamGroup), I32, I32, ctypes.c_float, ctypes.c_float, P],
+        "aniso_b200_loss_work_floats": [I32, I32, ctypes.POINTER(I64)],
+        "aniso_b200_loss_forward": [P, P, I32, I32, P, ctypes.c_float, ctypes.c_float, P, P, P],
+        "aniso_b200_loss_backward": [P, P, I32, I32, P, ctypes.c_float, P, P, P, P],
         "aniso_b200_render": [P, ctypes.POINTER(Camera), ctypes.POINTER(Options), P, ctypes.POINTER(Stats)],
         "aniso_b200_render_device": [P, ctypes.POINTER(Camera), ctypes.POINTER(Options), P, P],
         "aniso_b200_sync": [P, ctypes.POINTER(Stats)],

@@ -267,6 +267,21 @@ typedef struct aniso_b200_adam_group {
 int aniso_b200_adam_step(const aniso_b200_adam_group* groups, int32_t n_groups, int32_t step, float beta1,
                          float beta2, void* stream);
 
+/* The loss of the training loop (pipeline/train_gsplat.py:94-109, 178-180) and its gradient:
+ *   l1_weight mean|image - target| + ssim_weight (1 - mean SSIM(image, target)),
+ * SSIM over the whole positions of an 11x11 window. image, target and grad are DEVICE arrays of
+ * height*width*3 floats (11 to 32767 pixels a side), window 121 HOST floats, work a DEVICE array of
+ * *floats floats (8-byte aligned) that the forward fills for the backward, loss and upstream
+ * (dL/d(loss)) one DEVICE float each. Deterministic; the gradient rounds as the loss composed from
+ * tensor operations does. Enqueued on `stream`. */
+int aniso_b200_loss_work_floats(int32_t height, int32_t width, int64_t* floats);
+int aniso_b200_loss_forward(const float* image, const float* target, int32_t height, int32_t width,
+                            const float* window, float l1_weight, float ssim_weight, float* work, float* loss,
+                            void* stream);
+int aniso_b200_loss_backward(const float* image, const float* target, int32_t height, int32_t width,
+                             const float* window, float l1_weight, const float* work, const float* upstream,
+                             float* grad, void* stream);
+
 /* ---- introspection used by the parity tests (no counterpart in gpu_render.h) ---------------- */
 
 /* Runs the projection only and copies, per Gaussian, what the reference preprocess kernel
