@@ -7,10 +7,17 @@
 //   v = b2 v + (1 - b2) g g
 //   p = p - (lr / (1 - b1^t)) m / (sqrt(v) / sqrt(1 - b2^t) + eps)
 // with the bias corrections formed on the host in double, as torch does.
+//
+// Bound by memory: 16 bytes read and 12 written per parameter. A block takes kBlockElems elements of
+// one group, each thread two 16-byte words of each of the four arrays, all eight loads in flight
+// before the first use; a group whose arrays are not 16-byte aligned, and a group's last, partial
+// block, go element by element. Measured at 43.7M parameters (740k Gaussians): 302 us when every
+// element searched its group and divided a 64-bit index, 175 us now (6.97 TB/s of 28 bytes each).
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 #include <string>
 
@@ -24,41 +31,89 @@ namespace {
 
 constexpr int kMaxGroups = 8;
 
+constexpr int kThreads = 256;
+constexpr int kVecs = 2;  // 16-byte words per thread and array
+constexpr unsigned kBlockElems = kThreads * 4 * kVecs;
+
 struct AdamGroupDev {
     float* param;
     const float* grad;
     float* m;
     float* v;
-    unsigned long long begin;  // first element of this group in the concatenated index space
+    unsigned long long count;
+    unsigned first_block;             // the group's first block
     float step_size, step_size_head;  // lr / (1 - b1^t) for the row's tail and head
     float eps;
     int row, head;                    // floats per row; leading floats of a row that use the head rate
+    int aligned;                      // all four arrays are 16-byte aligned
 };
 
 struct AdamArgs {
     AdamGroupDev g[kMaxGroups];
     int n_groups;
-    unsigned long long total;
     float b1c, b2, b2c;  // 1 - b1, b2, 1 - b2
     float bc2_sqrt;      // sqrt(1 - b2^t)
 };
 
-__global__ void __launch_bounds__(256) adam_kernel(AdamArgs a) {
-    for (unsigned long long e = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x; e < a.total;
-         e += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
-        int k = 0;
-        while (k + 1 < a.n_groups && a.g[k + 1].begin <= e) ++k;
-        const AdamGroupDev& G = a.g[k];
-        const unsigned long long i = e - G.begin;
-        const float g = G.grad[i];
-        const float m = fmaf(a.b1c, g - G.m[i], G.m[i]);
-        const float v = fmaf(a.b2c, g * g, a.b2 * G.v[i]);
-        G.m[i] = m;
-        G.v[i] = v;
-        const bool in_head = G.head > 0 && static_cast<int>(i % static_cast<unsigned long long>(G.row)) < G.head;
-        const float step_size = in_head ? G.step_size_head : G.step_size;
-        const float denom = sqrtf(v) / a.bc2_sqrt + G.eps;
-        G.param[i] = fmaf(-step_size, m / denom, G.param[i]);
+__device__ __forceinline__ void adam_element(const AdamArgs& a, float step_size, float eps, float g, float& p, float& m,
+                                             float& v) {
+    m = fmaf(a.b1c, g - m, m);
+    v = fmaf(a.b2c, g * g, a.b2 * v);
+    const float denom = sqrtf(v) / a.bc2_sqrt + eps;
+    p = fmaf(-step_size, m / denom, p);
+}
+
+// Where element i sits in its row of `row` floats (64-bit division only past 2^32 elements).
+__device__ __forceinline__ unsigned row_place(unsigned long long i, int row) {
+    return i >> 32 ? static_cast<unsigned>(i % static_cast<unsigned>(row))
+                   : static_cast<unsigned>(i) % static_cast<unsigned>(row);
+}
+
+__global__ void __launch_bounds__(kThreads) adam_kernel(AdamArgs a) {
+    int k = 0;
+    while (k + 1 < a.n_groups && a.g[k + 1].first_block <= blockIdx.x) ++k;
+    const AdamGroupDev& G = a.g[k];
+    const unsigned long long base = static_cast<unsigned long long>(blockIdx.x - G.first_block) * kBlockElems;
+    if (!G.aligned || base + kBlockElems > G.count) {
+        for (unsigned e = threadIdx.x; e < kBlockElems && base + e < G.count; e += kThreads) {
+            const unsigned long long i = base + e;
+            float p = G.param[i], m = G.m[i], v = G.v[i];
+            const bool in_head = G.head > 0 && row_place(i, G.row) < static_cast<unsigned>(G.head);
+            adam_element(a, in_head ? G.step_size_head : G.step_size, G.eps, G.grad[i], p, m, v);
+            G.param[i] = p;
+            G.m[i] = m;
+            G.v[i] = v;
+        }
+        return;
+    }
+    float4 g[kVecs], p[kVecs], m[kVecs], v[kVecs];
+#pragma unroll
+    for (int u = 0; u < kVecs; ++u) {
+        const unsigned long long i = base + (u * kThreads + threadIdx.x) * 4u;
+        g[u] = *reinterpret_cast<const float4*>(G.grad + i);
+        p[u] = *reinterpret_cast<const float4*>(G.param + i);
+        m[u] = *reinterpret_cast<const float4*>(G.m + i);
+        v[u] = *reinterpret_cast<const float4*>(G.v + i);
+    }
+#pragma unroll
+    for (int u = 0; u < kVecs; ++u) {
+        const unsigned long long i = base + (u * kThreads + threadIdx.x) * 4u;
+        float step[4] = {G.step_size, G.step_size, G.step_size, G.step_size};
+        if (G.head > 0) {
+            unsigned r = row_place(i, G.row);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (r < static_cast<unsigned>(G.head)) step[e] = G.step_size_head;
+                if (++r == static_cast<unsigned>(G.row)) r = 0;
+            }
+        }
+        adam_element(a, step[0], G.eps, g[u].x, p[u].x, m[u].x, v[u].x);
+        adam_element(a, step[1], G.eps, g[u].y, p[u].y, m[u].y, v[u].y);
+        adam_element(a, step[2], G.eps, g[u].z, p[u].z, m[u].z, v[u].z);
+        adam_element(a, step[3], G.eps, g[u].w, p[u].w, m[u].w, v[u].w);
+        *reinterpret_cast<float4*>(G.param + i) = p[u];
+        *reinterpret_cast<float4*>(G.m + i) = m[u];
+        *reinterpret_cast<float4*>(G.v + i) = v[u];
     }
 }
 
@@ -78,7 +133,7 @@ extern "C" int aniso_b200_adam_step(const aniso_b200_adam_group* groups, int32_t
     a.b2 = beta2;
     a.b2c = 1.0f - beta2;
     a.bc2_sqrt = static_cast<float>(std::sqrt(bc2));
-    unsigned long long total = 0;
+    unsigned long long blocks = 0;
     for (int k = 0; k < n_groups; ++k) {
         const aniso_b200_adam_group& s = groups[k];
         if (s.count < 0 || (s.count > 0 && (!s.param || !s.grad || !s.exp_avg || !s.exp_avg_sq)))
@@ -90,18 +145,21 @@ extern "C" int aniso_b200_adam_step(const aniso_b200_adam_group* groups, int32_t
         d.grad = s.grad;
         d.m = s.exp_avg;
         d.v = s.exp_avg_sq;
-        d.begin = total;
+        d.count = static_cast<unsigned long long>(s.count);
+        d.first_block = static_cast<unsigned>(blocks);
+        d.aligned = ((reinterpret_cast<uintptr_t>(s.param) | reinterpret_cast<uintptr_t>(s.grad) |
+                      reinterpret_cast<uintptr_t>(s.exp_avg) | reinterpret_cast<uintptr_t>(s.exp_avg_sq)) & 15) == 0;
         d.step_size = static_cast<float>(static_cast<double>(s.lr) / bc1);
         d.step_size_head = static_cast<float>(static_cast<double>(s.head > 0 ? s.lr_head : s.lr) / bc1);
         d.eps = s.eps;
         d.row = s.row > 0 ? s.row : 1;
         d.head = s.head;
-        total += static_cast<unsigned long long>(s.count);
+        blocks += (d.count + kBlockElems - 1) / kBlockElems;
+        if (blocks > 0x7FFFFFFFull)
+            return ab2::report_error(ANISO_B200_ERR_ARGUMENT, "too many elements for one Adam launch");
     }
-    a.total = total;
-    if (total == 0) return ANISO_B200_OK;
-    const unsigned long long blocks = std::min<unsigned long long>((total + 255) / 256, 148ull * 16);
-    adam_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+    if (blocks == 0) return ANISO_B200_OK;
+    adam_kernel<<<static_cast<unsigned>(blocks), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return ab2::report_error(ANISO_B200_ERR_CUDA, cudaGetErrorString(e));
     return ANISO_B200_OK;
