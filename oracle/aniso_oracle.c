@@ -293,7 +293,7 @@ int orc_render(int64_t n, const float* gauss, const float* sh, int scene_degree,
                     const float power = -0.5f * (s->A * dx * dx + s->C * dy * dy) - s->B * dx * dy;
                     if (power > 0) continue;
                     const float e = s->opacity * expf(power);
-                    const float alpha = 0.99f < e ? 0.99f : e; /* std::min(0.99f, e) */
+                    const float alpha = e < 0.99f ? e : 0.99f; /* std::min(0.99f, e): 0.99 for a NaN */
                     if (alpha < 1.0f / 255.0f) continue;
                     const float next_t = T * (1 - alpha);
                     if (next_t < 1e-4f) break;
