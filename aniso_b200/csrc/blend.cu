@@ -7,28 +7,31 @@
 //   stop (without applying) once T (1 - alpha) < 1e-4; else C += rgb alpha T, T *= 1 - alpha
 // evaluated in base 2 on the pre-scaled conic of the SplatRecord (one MUFU ex2 per evaluation).
 //
-// B200 mapping (the kernel is FP32-issue bound, so the layout minimises instructions per pixel):
-//   * each warp owns one 8x8 pixel block -- exactly one tile of the CPU renderer -- with two
+// B200 mapping (the kernel is issue bound, its ALU pipe the busiest, so the layout minimises
+// instructions per pixel):
+//   * each warp owns one 8x8 pixel block, each quarter warp one of its 4x4 cells, with two
 //     horizontally adjacent pixels per lane; the row terms of the exponent (with log2(opacity)
 //     folded in) are shared, and the two pixels' offsets and FMAs are packed FP32x2 instructions
 //     (three for both pixels' exponents);
 //   * the block stages kBatch splat records per round in shared memory and, per splat, a mask of
-//     the warp blocks it can touch (staged_block_mask): its pixel bounds (the CPU 8x8-tile
+//     the tile's cells it can touch (staged_cell_mask): its pixel bounds (the CPU 8x8-tile
 //     rectangle cut by the bounding box of the ellipse where alpha can reach 1/255, with a margin)
-//     against each 8x8 block -- which gives every pixel exactly the splat list of the CPU renderer
-//     whatever the tile shape (so the image does not depend on it) -- and, in training, the
-//     record's block bits (the blocks where the ellipse itself reaches the cut, set once per splat
-//     by the training preprocess), which only drop splats that cannot pass the alpha test anywhere
-//     in the block, so they change no result. The plain forward leaves them out: their cost in the
-//     preprocess (+14 us per 740k frame) is more than the blend steps they save (-9 us), where the
-//     training step, whose adjoint replays every step at about four times the cost, gains (forward
-//     and adjoint at 2.2M: 1.84 -> 1.73 ms; the 8-scene training batch 29.0 -> 27.0 ms a step).
-//     Testing every block against the ellipse in each tile's staging instead cost more than it
-//     saved: 0.161 -> 0.186 ms of blend;
-//   * each warp walks only its splats (listed once per round from the masks by ballot and
-//     popcount); a finished pixel holds T = 0 (T >= 1e-4 while it is not finished), so no
-//     separate flag is carried; the warp leaves once all 64 pixels are finished and the block
-//     stops loading once all its warps have (__syncthreads_or).
+//     and the ellipse itself -- splats that are left out could not pass the alpha test anywhere in
+//     the cell, so every pixel takes the splat list of the CPU renderer whatever the tile shape;
+//   * each quarter warp walks only its own cell's splats (listed once per round from the masks by
+//     ballot and popcount), the four side by side: a splat costs a warp a step only as often as its
+//     quarters need it, and 4x4 cells waste fewer pixels around a splat than 8x8 blocks. The
+//     quarters meet at the end of a round, so longer rounds even out their lists. Measured per 740k
+//     1280x720 frame: blend 139 -> 124 us (122.7M -> 96.3M warp instructions) with one list per
+//     quarter instead of per warp, the frame 266 -> 259 us with 256-splat rounds instead of 128,
+//     -> 253 us with the ellipse test (8x8 blocks against the ellipse, in each tile's staging, had
+//     cost more than they saved);
+//   * a finished pixel holds T = 0 (T >= 1e-4 while it is not finished), so no separate flag is
+//     carried; the warp leaves once all 64 pixels are finished and the block stops loading once all
+//     its warps have (__syncthreads_or).
+// Tried and slower: comparisons as 0 / 1 floats with packed products in place of the selects
+// (+1.5% per frame), predicated scalar updates (+4%), operands staged in pairs (+5.5%), ten CTAs per
+// SM by holding the kernel to 48 registers (+3%).
 #include "common.cuh"
 #include "kernels.h"
 
@@ -130,25 +133,35 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_kernel(const uint2* __restr
     chain_entry();
     constexpr int kThreads = TW * TH / 2;  // two pixels per lane
     constexpr int kWarpsX = TW / 8;
-    __shared__ float4 s_r0[kBatch];
-    __shared__ float4 s_r1[kBatch];
-    __shared__ float s_b[kBatch];
-    __shared__ unsigned char s_mask[kBatch];
-    __shared__ unsigned short s_list[kThreads / 32][kBatch];  // each warp's splats of the round
+    constexpr int kCells = TW / 4;         // 4x4-pixel cells per tile row
+    __shared__ float4 s_r0[kBatch + 1];    // the last slot: a splat that no pixel takes
+    __shared__ float4 s_r1[kBatch + 1];
+    __shared__ float s_b[kBatch + 1];
+    __shared__ unsigned s_mask[kBatch];
+    __shared__ __align__(8) unsigned short s_list[kThreads / 8][kBatch + 4];  // each quarter warp's splats of the round
     __shared__ __align__(16) unsigned char s_px[TH * TW * 3];  // the tile's RGB8, staged for row stores
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quarter = lane >> 3;
     const unsigned gtile = blockIdx.x;
     const unsigned v = find_segment(tables.tile_base, tables.n_views, gtile);
     const ViewInfo& vi = views[v];
     const int tiles_x = vi.cam.tilesX;
     const unsigned local = gtile - vi.tile_base;
     const int ox = static_cast<int>(local % tiles_x) * TW, oy = static_cast<int>(local / tiles_x) * TH;
-    const int x0 = ox + (warp % kWarpsX) * 8 + 2 * (lane & 3), y = oy + (warp / kWarpsX) * 8 + (lane >> 2);
+    const int x0 = ox + (warp % kWarpsX) * 8 + 4 * (quarter & 1) + 2 * (lane & 1);
+    const int y = oy + (warp / kWarpsX) * 8 + 4 * (quarter >> 1) + ((lane >> 1) & 3);
     const int width = vi.cam.width, height = vi.cam.height;
     const float px0 = x0 + 0.5f, py = y + 0.5f;
     const uint2 range = (ctrl->flags & kFlagOverflow) ? make_uint2(0, 0) : ranges[gtile];
     const unsigned lt = lanemask_lt();
+    // The warp's cells in a staged splat's mask: quarters 0 and 1 at this bit, 2 and 3 one row below.
+    const int cell0 = (warp / kWarpsX) * 2 * kCells + (warp % kWarpsX) * 2;
+
+    if (tid == 0) {
+        s_r0[kBatch] = make_float4(0.f, 0.f, 0.f, 0.f);
+        s_r1[kBatch] = make_float4(0.f, -INFINITY, 0.f, 0.f);
+        s_b[kBatch] = 0.f;
+    }
 
     // Pixels outside the image start finished.
     float2 T = make_float2((x0 < width && y < height) ? 1.0f : 0.f, (x0 + 1 < width && y < height) ? 1.0f : 0.f);
@@ -169,38 +182,46 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_kernel(const uint2* __restr
                 s_r0[slot] = r.r0;
                 s_r1[slot] = make_float4(r.r1.x, r.r1.y, fminf(r.r1.z, kMax), fminf(r.r1.w, kMax));
                 s_b[slot] = fminf(r.r2.x, kMax);
-                m = staged_block_mask<TW, TH, kTrain>(r, ox, oy);
+                m = staged_cell_mask<TW, TH>(r, ox, oy);
             }
-            s_mask[slot] = static_cast<unsigned char>(m);
+            s_mask[slot] = m;
         }
         __syncthreads();
         const unsigned cnt = min(static_cast<unsigned>(kBatch), range.y - base);
-        if (!__any_sync(0xFFFFFFFFu, T.x + T.y > 0.f)) continue;  // the warp is finished
-        // The warp's splats of the round in list order, compacted once (a ballot per 32 staged)
-        // rather than found bit by bit in each step (0.1395 -> 0.1376 ms per 740k frame).
-        unsigned n = 0;
+        const unsigned live = __ballot_sync(0xFFFFFFFFu, T.x + T.y > 0.f);
+        if (!live) continue;  // the warp is finished
+        // Each quarter's splats of the round in list order, compacted once (a ballot per quarter and 32
+        // staged); a finished quarter takes none. Then every list is padded with the splat that no
+        // pixel takes to the longest one's length, a multiple of four.
+        unsigned n[4] = {0, 0, 0, 0};
         for (unsigned c = 0; c * 32 < cnt; ++c) {
             const unsigned idx = c * 32 + lane;
-            const bool mine = idx < cnt && ((s_mask[idx] >> warp) & 1u);
-            const unsigned bits = __ballot_sync(0xFFFFFFFFu, mine);
-            if (mine) s_list[warp][n + __popc(bits & lt)] = static_cast<unsigned short>(idx);
-            n += __popc(bits);
+            const unsigned m = idx < cnt ? s_mask[idx] >> cell0 : 0u;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const bool mine = ((live >> (8 * q)) & 0xFFu) && ((m >> ((q & 1) + (q >> 1) * kCells)) & 1u);
+                const unsigned bits = __ballot_sync(0xFFFFFFFFu, mine);
+                if (mine) s_list[warp * 4 + q][n[q] + __popc(bits & lt)] = static_cast<unsigned short>(idx);
+                n[q] += __popc(bits);
+            }
         }
+        const unsigned longest = (max(max(n[0], n[1]), max(n[2], n[3])) + 3u) & ~3u;
+        const unsigned short* list = s_list[warp * 4 + quarter];
+        const unsigned own = quarter == 0 ? n[0] : quarter == 1 ? n[1] : quarter == 2 ? n[2] : n[3];
+        for (unsigned i = own + (lane & 7); i < longest; i += 8) s_list[warp * 4 + quarter][i] = kBatch;
         __syncwarp();
-        for (unsigned i = 0; i < n; i += 4) {
-            // Up to four splats per vote on whether the warp is finished (a vote per splat, or per
-            // two, costs more than the steps a finished warp walks in vain: 0.161 -> 0.154 ms per
-            // 740k frame from two to four).
+        for (unsigned i = 0; i < longest; i += 4) {
+            const ushort4 four = *reinterpret_cast<const ushort4*>(list + i);
+            const unsigned id[4] = {four.x, four.y, four.z, four.w};
+            // Four splats per vote on whether the warp is finished.
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                if (i + u >= n) break;
-                const unsigned jj = s_list[warp][i + u];
-                const float4 a = s_r0[jj];
-                const float4 k = s_r1[jj];
-                const float bb = s_b[jj];
+                const float4 a = s_r0[id[u]];
+                const float4 k = s_r1[id[u]];
+                const float bb = s_b[id[u]];
                 float2 dx;
                 const float2 pp = splat_exponents2(a, k, make_float2(px0, px0 + 1.0f), __fsub_rn(py, a.y), dx);
-                blend_px2<kTrain>(pp, k.y, k.z, k.w, bb, T, cr, cg, cb, tf, last0, last1, base + jj + 1);
+                blend_px2<kTrain>(pp, k.y, k.z, k.w, bb, T, cr, cg, cb, tf, last0, last1, base + id[u] + 1);
             }
             if (!__any_sync(0xFFFFFFFFu, T.x + T.y > 0.f)) break;
         }
@@ -246,7 +267,7 @@ void launch_blend(unsigned tiles, const uint2* ranges, const unsigned* sorted_va
         if (big) launch_shape<8, 8, 256>(tiles, ranges, sorted_vals, rec, ctrl, views, tables, train, stream);
         else launch_shape<8, 8, 128>(tiles, ranges, sorted_vals, rec, ctrl, views, tables, train, stream);
     } else if (tile_h == 32) {
-        if (big) launch_shape<16, 32, 512>(tiles, ranges, sorted_vals, rec, ctrl, views, tables, train, stream);
+        if (big) launch_shape<16, 32, 256>(tiles, ranges, sorted_vals, rec, ctrl, views, tables, train, stream);
         else launch_shape<16, 32, 256>(tiles, ranges, sorted_vals, rec, ctrl, views, tables, train, stream);
     } else {
         if (big) launch_shape<16, 16, 256>(tiles, ranges, sorted_vals, rec, ctrl, views, tables, train, stream);

@@ -382,11 +382,11 @@ int pack_camera(int scene_degree, int rendered_degree, const aniso_b200_camera* 
 
 // ---- plans ---------------------------------------------------------------------------------
 
-// Launch shape of a plan. A single-view render uses 16x16 tiles (the reference's) and 128-splat
-// blend rounds (measured 0.321 against 0.325 ms per 740k frame with 256); batches take theirs from
-// their options (the autotuner's choice).
+// Launch shape of a plan. A single-view render uses 16x16 tiles (the reference's) and 256-splat
+// blend rounds (measured 0.259 against 0.266 ms per 740k frame with 128, 0.548 against 0.563 ms at
+// 2.2M and 1920x1080); batches take theirs from their options (the autotuner's choice).
 struct PlanShape {
-    int tile_w = kTile, tile_h = kTile, blend_batch = 128, sh_degree = 3, radix_bits = kRadixBits;
+    int tile_w = kTile, tile_h = kTile, blend_batch = 256, sh_degree = 3, radix_bits = kRadixBits;
     float splat_scale = 1.0f;
     bool use_graph = false;
 };

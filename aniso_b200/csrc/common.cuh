@@ -427,4 +427,64 @@ __device__ __forceinline__ unsigned staged_block_mask(const SplatRecord& r, int 
     return m;
 }
 
+// The 4x4-pixel cells of a TW x TH tile at pixel (ox, oy, multiples of 8) that a staged splat record
+// may touch, bit rr * (TW / 4) + c for cell (c, rr): the cells its pixel bounds overlap, less those
+// where its exponent stays below log2(1/255) at every pixel centre (no pixel there could take
+// anything from it, so leaving them out changes no result and the image does not depend on the tile
+// shape). The test, per row of cells, is on the x-extent of the ellipse where the exponent reaches
+// the cut, over the band of the row's centre offsets: the form A x^2 + B x y + C y^2 is concave
+// (A, C < 0, 4AC > B^2), so the ellipse's right boundary is concave in y, largest (the half-width W) at
+// y = yr = -B W / 2C; over a band it is largest at the band's point nearest yr, where x is the larger
+// root of the quadratic in x, of discriminant (B^2 - 4AC) y^2 + 4AD. The left boundary likewise,
+// mirrored (y = -yr). Where that point has no root, the band misses the ellipse.
+//
+// Conservative: the cut is lowered by 0.02 plus a term relative to the size of the form's terms over
+// the bounds (in log2 units: far above the rounding of this test and of the blend's evaluation, also
+// for needles, whose terms cancel), and the extent is widened by 1e-3 of the half-width plus 0.01
+// pixel (MUFU square roots and reciprocals, relative error ~2^-22). A degenerate form (a coefficient
+// that is 0 or not finite, or not concave) keeps every cell of the bounds.
+template <int TW, int TH>
+__device__ __forceinline__ unsigned staged_cell_mask(const SplatRecord& r, int ox, int oy) {
+    constexpr float kCut = -7.99435343685885793f;  // log2(1/255)
+    constexpr int kC = TW / 4, kR = TH / 4;
+    static_assert(kC * kR <= 32, "one bit per cell");
+    const unsigned bx = __float_as_uint(r.r2.y), by = __float_as_uint(r.r2.z);
+    const int xlo = unpack_lo(bx), xhi = unpack_hi(bx), ylo = unpack_lo(by), yhi = unpack_hi(by);
+    unsigned cols = 0, m = 0;
+#pragma unroll
+    for (int c = 0; c < kC; ++c)
+        if (xlo <= ox + 4 * c + 3 && xhi >= ox + 4 * c) cols |= 1u << c;
+#pragma unroll
+    for (int rr = 0; rr < kR; ++rr)
+        if (ylo <= oy + 4 * rr + 3 && yhi >= oy + 4 * rr) m |= cols << (kC * rr);
+
+    const float u = r.r0.x, v = r.r0.y, A = r.r0.z, B = r.r0.w, C = r.r1.x, L = r.r1.y;
+    const float det4 = 4.f * A * C - B * B;
+    if (!(A < 0.f && C < 0.f && det4 > 0.f && isfinite(A + B + C + L + det4))) return m;
+    const float mx = fmaxf(fabsf(xlo + 0.5f - u), fabsf(xhi + 0.5f - u));
+    const float my = fmaxf(fabsf(ylo + 0.5f - v), fabsf(yhi + 0.5f - v));
+    const float size = fabsf(A) * mx * mx + fabsf(B) * mx * my + fabsf(C) * my * my;
+    const float D = kCut - 0.02f - 1e-5f * size - L;  // the form must reach D somewhere
+    if (D > 0.f) return 0u;                           // it cannot: its largest value is 0
+    const float W = sqrt_mufu(D * (4.f * C) * __frcp_rn(det4));  // half-width: D / (A - B^2 / 4C)
+    const float yr = -B * W * __frcp_rn(2.f * C);
+    const float inv2a = __frcp_rn(2.f * A);
+    const float eps = 1e-3f * W + 0.01f;
+    const float ad4 = 4.f * A * D, centre = u - static_cast<float>(ox);
+    unsigned keep = 0;
+#pragma unroll
+    for (int rr = 0; rr < kR; ++rr) {
+        const float Y0 = static_cast<float>(oy + 4 * rr) + 0.5f - v, Y1 = Y0 + 3.f;
+        const float ya = fminf(fmaxf(yr, Y0), Y1), yb = fminf(fmaxf(-yr, Y0), Y1);
+        const float da = fmaf(-det4 * ya, ya, ad4), db = fmaf(-det4 * yb, yb, ad4);
+        const float xr = (-sqrt_mufu(fmaxf(da, 0.f)) - B * ya) * inv2a;
+        const float xl = (sqrt_mufu(fmaxf(db, 0.f)) - B * yb) * inv2a;
+        // cells whose centre offsets [4 c + 0.5, 4 c + 3.5] (from ox) meet [xl - eps, xr + eps]
+        const int lo = max(0, __float2int_ru((centre + xl - eps - 3.5f) * 0.25f));
+        const int hi = min(kC - 1, __float2int_rd((centre + xr + eps - 0.5f) * 0.25f));
+        if (da >= 0.f && db >= 0.f && lo <= hi) keep |= ((2u << hi) - (1u << lo)) << (kC * rr);
+    }
+    return m & keep;
+}
+
 }  // namespace ab2

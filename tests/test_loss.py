@@ -34,7 +34,7 @@ def test_loss_and_gradient_match_64_bits(height, width):
     (want_grad,) = torch.autograd.grad(3.0 * want, x)
     # Variances are differences of fp32 sums near 1: absolute error about 2^-22 against B2 >= 9e-4, so
     # relative errors of a window's terms stay below 3e-4 and, over the image, far below.
-    assert abs(float(loss) - float(want)) <= 1e-5
+    assert abs(loss.item() - float(want)) <= 1e-5
     assert float((grad.double() - want_grad).norm() / want_grad.norm()) <= 3e-4
 
     # And bit for bit the gradient of the loss composed from tensor operations.
