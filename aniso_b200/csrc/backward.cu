@@ -1,16 +1,21 @@
 // The adjoint of the rasterizer (no counterpart in the reference, which has no backward pass; the
 // forward it differentiates is render.cpp:39-104 / 195-220 on the GPU path's lists).
 //
-// blend_backward: one block per tile of a batch, the forward's pixel layout (8x8 per warp, two
-//   pixels per lane). Each pixel walks its tile list back to front from its last applied
-//   splat, replaying the forward's alpha tests bit for bit (same record, same exponent code) and
+// blend_backward: one block per tile of a batch; a warp owns an 8x8 block, each quarter warp two of its
+//   columns, with two pixels per lane. Each pixel walks its tile list back to front from its last
+//   applied splat, replaying the forward's alpha tests bit for bit (same record, same exponent code) and
 //   recovering the transmittance in front of each splat (T_j = T_{j+1} / (1 - a_j));
-//   nothing per pixel is stored but the final T and the last contributor. Per splat, the gradient
-//   with respect to its nine record parameters (u, v, A2, B2, C2, L, r, g, b) is reduced over the
-//   warp (12 shuffles for the 9 values; skipped when no pixel of the warp took the splat), summed
-//   over the warps in a fixed order, and written
-//   to the pair's slot in the depth-ordered pair list -- no atomics, so the result does not depend
-//   on scheduling.
+//   nothing per pixel is stored but the final T and the last contributor. As in the forward, each
+//   quarter walks only the splats its own cell (2x8 pixels) can take, the four side by side. Per splat
+//   and cell, the gradient with respect to the nine record parameters (u, v, A2, B2, C2, L, r, g, b)
+//   is summed over the quarter's lanes (through shared memory: half the instructions of shuffling
+//   nine values), and at the end of a round over the quarters and warps, all in a fixed order, and
+//   written to the pair's slot in the pair list -- no atomics, so the result does not depend on
+//   scheduling, and the sums are those of the whole warp's butterfly, bit for bit.
+//   Bound by issue (2.65 of 4 instructions a cycle, every pipe below 40%) at the 24 warps per SM that
+//   the sums' shared memory leaves. Measured at 2.2M / 1280x720: 647 us with one list per warp and
+//   warp-wide shuffles, 587 us with lists per quarter, 569 us with the sums through shared memory and
+//   room for 512 of them (6 CTAs per SM; 640 and 768: 585 us).
 // gauss_backward: one launch per view over the Gaussians visible in it (compacted first, so no lane
 //   idles on a culled one); each sums its pairs' slots (contiguous, in a fixed order), applies the
 //   chain rule through the record
@@ -18,6 +23,8 @@
 //   transform), the 3D covariance M M^T with M = R(q) diag(s), and the activations (exp, sigmoid,
 //   quaternion normalisation) to the 59 raw parameters, and adds them to the scene's gradients.
 //   Views are launched one after another, so the sum over views also runs in a fixed order.
+#include <atomic>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -25,42 +32,11 @@ namespace ab2 {
 namespace {
 
 constexpr int kBatch = 128;
+constexpr int kBackwardPlaces = 512;  // (splat, cell) sums a 16x16 tile's round has room for
 constexpr int kG = 9;
 constexpr float kLn2 = 0.69314718055994530942f;
 constexpr float kHalfLog2e = -0.72134752044448170368f;  // A2 = kHalfLog2e * A, C2 likewise
 constexpr float kNegLog2e = -1.44269504088896340736f;   // B2 = kNegLog2e * B
-
-// Sums v[0..8] over the warp; afterwards the even lanes hold one sum each: value index *k (-1 for
-// none). 12 shuffles: each step hands half of the values to the partner lane.
-__device__ __forceinline__ float warp_reduce9(const float v[kG], int lane, int& k) {
-    const bool b16 = lane & 16, b8 = lane & 8, b4 = lane & 4, b2 = lane & 2;
-    float a[5];
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-        const float lo = v[i], hi = i + 5 < kG ? v[i + 5] : 0.f;
-        a[i] = (b16 ? hi : lo) + __shfl_xor_sync(0xFFFFFFFFu, b16 ? lo : hi, 16);
-    }
-    float b[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const float lo = a[i], hi = i + 3 < 5 ? a[i + 3] : 0.f;
-        b[i] = (b8 ? hi : lo) + __shfl_xor_sync(0xFFFFFFFFu, b8 ? lo : hi, 8);
-    }
-    float c[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const float lo = b[i], hi = i + 2 < 3 ? b[i + 2] : 0.f;
-        c[i] = (b4 ? hi : lo) + __shfl_xor_sync(0xFFFFFFFFu, b4 ? lo : hi, 4);
-    }
-    const float d = (b2 ? c[1] : c[0]) + __shfl_xor_sync(0xFFFFFFFFu, b2 ? c[0] : c[1], 2);
-    const float e = d + __shfl_xor_sync(0xFFFFFFFFu, d, 1);
-    const int ci = b2 ? 1 : 0;
-    const int bi = ci + (b4 ? 2 : 0);
-    const int ai = bi + (b8 ? 3 : 0);
-    const int vi = ai + (b16 ? 5 : 0);
-    k = ((lane & 1) == 0 && bi < 3 && ai < 5 && vi < kG) ? vi : -1;
-    return e;
-}
 
 __device__ __forceinline__ float rcp_approx(float x) {
     float y;
@@ -76,32 +52,38 @@ struct PixelState2 {
     unsigned last0, last1;    // list position one past each pixel's last applied splat
 };
 
-// One adjoint step for splat j (list position pos) at both pixels of the lane, each pair of
-// operations one packed FP32x2 instruction (sm_100; per component the rounding of the scalar
-// form). A pixel the splat does not apply to in the forward (behind its last applied splat, or
-// failing the alpha tests, replayed with the forward's exponent bits) takes alpha = 0, which
-// leaves its state unchanged (1/(1 - 0) = 1, w = 0) and adds zeros. G[k] receives the two pixels'
-// gradients of the nine record parameters (u, v, A2, B2, C2, L, r, g, b); the caller adds the
-// halves. Returns whether the splat applied to either pixel. 1/(1 - alpha) is the approximate
-// reciprocal (relative error below 2^-22): the recovered transmittance drifts by that much per
-// splat, far inside the gradients' tolerance. Packing the two pixels took the fwd+bwd of the
-// 2.2M-Gaussian view from 1.95 to 1.86 ms.
+// The exponentials and whether the splat at list position pos applied in the forward to each of the
+// lane's pixels (not behind its last applied splat, and passing the alpha tests, replayed with the
+// forward's exponent bits).
+struct PixelTest2 {
+    float e0, e1;
+    bool v0, v1;
+};
+__device__ __forceinline__ PixelTest2 pixel_test2(const PixelState2& s, unsigned pos, float2 p, float L) {
+    PixelTest2 t;
+    t.e0 = ex2_approx(p.x);
+    t.e1 = ex2_approx(p.y);
+    t.v0 = pos < s.last0 && !(p.x > L) && fminf(0.99f, t.e0) >= 1.0f / 255.0f;
+    t.v1 = pos < s.last1 && !(p.y > L) && fminf(0.99f, t.e1) >= 1.0f / 255.0f;
+    return t;
+}
 
-__device__ __forceinline__ bool pixel_step2(PixelState2& s, unsigned pos, float2 p, float2 dx, float dy,
-                                            const float4& r0, const float4& r1, float rb, float2 G[kG]) {
-    const float e0 = ex2_approx(p.x), e1 = ex2_approx(p.y);
-    const float a0 = fminf(0.99f, e0), a1 = fminf(0.99f, e1);
-    const bool v0 = pos < s.last0 && !(p.x > r1.y) && a0 >= 1.0f / 255.0f;
-    const bool v1 = pos < s.last1 && !(p.y > r1.y) && a1 >= 1.0f / 255.0f;
-    if (!(v0 || v1)) return false;
-    const float2 alpha = make_float2(v0 ? a0 : 0.f, v1 ? a1 : 0.f);
+// One adjoint step at both pixels of the lane, each pair of operations one packed FP32x2 instruction
+// (sm_100; per component the rounding of the scalar form). A pixel the splat did not apply to takes
+// alpha = 0, which leaves its state unchanged (1/(1 - 0) = 1, w = 0) and adds zeros, so every lane of
+// a warp with any such pixel takes the step without a branch. g[k] receives the gradients of the nine
+// record parameters (u, v, A2, B2, C2, L, r, g, b), the sum of the two pixels'. 1/(1 - alpha) is the
+// approximate reciprocal (relative error below 2^-22): the recovered transmittance drifts by that
+// much per splat, far inside the gradients' tolerance. Packing the two pixels took the fwd+bwd of
+// the 2.2M-Gaussian view from 1.95 to 1.86 ms.
+__device__ __forceinline__ void pixel_step2(PixelState2& s, const PixelTest2& t, float2 dx, float dy, const float4& r0,
+                                            const float4& r1, float rb, float g[kG]) {
+    const float2 alpha = make_float2(t.v0 ? fminf(0.99f, t.e0) : 0.f, t.v1 ? fminf(0.99f, t.e1) : 0.f);
     const float2 om = __fadd2_rn(make_float2(1.0f, 1.0f), make_float2(-alpha.x, -alpha.y));
     const float2 inv_om = make_float2(rcp_approx(om.x), rcp_approx(om.y));
     const float2 Tb = __fmul2_rn(s.T, inv_om);  // transmittance in front of the splat
     const float2 w = __fmul2_rn(alpha, Tb);
-    G[6] = __fmul2_rn(s.gr, w);
-    G[7] = __fmul2_rn(s.gg, w);
-    G[8] = __fmul2_rn(s.gb, w);
+    const float2 G6 = __fmul2_rn(s.gr, w), G7 = __fmul2_rn(s.gg, w), G8 = __fmul2_rn(s.gb, w);
     const float2 tr = __ffma2_rn(make_float2(r1.z, r1.z), Tb, __fmul2_rn(make_float2(-s.ar.x, -s.ar.y), inv_om));
     const float2 tg = __ffma2_rn(make_float2(r1.w, r1.w), Tb, __fmul2_rn(make_float2(-s.ag.x, -s.ag.y), inv_om));
     const float2 tb = __ffma2_rn(make_float2(rb, rb), Tb, __fmul2_rn(make_float2(-s.ab.x, -s.ab.y), inv_om));
@@ -110,48 +92,80 @@ __device__ __forceinline__ bool pixel_step2(PixelState2& s, unsigned pos, float2
     s.ag = __ffma2_rn(make_float2(r1.w, r1.w), w, s.ag);
     s.ab = __ffma2_rn(make_float2(rb, rb), w, s.ab);
     s.T = Tb;
-    // d alpha / d p = alpha ln 2 unless clamped (alpha = 0 for a pixel that takes no part)
+    // d alpha / d p = alpha ln 2 unless clamped or not applied
     float2 dp = __fmul2_rn(__fmul2_rn(dalpha, alpha), make_float2(kLn2, kLn2));
-    if (e0 > 0.99f) dp.x = 0.f;
-    if (e1 > 0.99f) dp.y = 0.f;
+    if (!t.v0 || t.e0 > 0.99f) dp.x = 0.f;
+    if (!t.v1 || t.e1 > 0.99f) dp.y = 0.f;
     const float2 ndp = make_float2(-dp.x, -dp.y);
     const float bdy = r0.w * dy, cdy2 = 2.0f * r1.x * dy;
-    G[0] = __fmul2_rn(ndp, __ffma2_rn(make_float2(2.0f * r0.z, 2.0f * r0.z), dx, make_float2(bdy, bdy)));
-    G[1] = __fmul2_rn(ndp, __ffma2_rn(make_float2(r0.w, r0.w), dx, make_float2(cdy2, cdy2)));
+    const float2 G0 = __fmul2_rn(ndp, __ffma2_rn(make_float2(2.0f * r0.z, 2.0f * r0.z), dx, make_float2(bdy, bdy)));
+    const float2 G1 = __fmul2_rn(ndp, __ffma2_rn(make_float2(r0.w, r0.w), dx, make_float2(cdy2, cdy2)));
     const float2 dpdx = __fmul2_rn(dp, dx);
-    G[2] = __fmul2_rn(dpdx, dx);
-    G[3] = __fmul2_rn(dpdx, make_float2(dy, dy));
-    G[4] = __fmul2_rn(dp, make_float2(dy * dy, dy * dy));
-    G[5] = dp;
-    return true;
+    const float2 G2 = __fmul2_rn(dpdx, dx);
+    const float2 G3 = __fmul2_rn(dpdx, make_float2(dy, dy));
+    const float2 G4 = __fmul2_rn(dp, make_float2(dy * dy, dy * dy));
+    g[0] = G0.x + G0.y;
+    g[1] = G1.x + G1.y;
+    g[2] = G2.x + G2.y;
+    g[3] = G3.x + G3.y;
+    g[4] = G4.x + G4.y;
+    g[5] = dp.x + dp.y;
+    g[6] = G6.x + G6.y;
+    g[7] = G7.x + G7.y;
+    g[8] = G8.x + G8.y;
 }
 
+constexpr int kRedPitch = 36;  // floats per value: a quarter's eight lanes as two 16-byte words, free of conflicts
+
+// Shared memory of one CTA. A quarter warp's sums for the splats of its list go to consecutive places
+// of grad; at[slot][list] is where a staged splat's sums of that list start (place kPlaces, which holds
+// zeros, where the list leaves the splat out).
+template <int TW, int TH>
+struct BackwardShared {
+    static constexpr int kLists = TW * TH / 16;           // quarter warps: cells of 2 x 8 pixels
+    static constexpr int kPlaces = TW * TH == 64 ? 4 * kBatch : TW * TH * kBackwardPlaces / 256;
+    float4 r0[kBatch + 1];                                // the last slot: a splat that no pixel takes
+    float4 r1[kBatch + 1];
+    unsigned short at[kBatch][kLists];
+    float grad[(kPlaces + 1) * kG];
+    float b[kBatch + 1];
+    unsigned pos[kBatch];
+    unsigned mask[kBatch];
+    unsigned char list[kLists][kBatch + 4];
+    __align__(16) float red[kLists / 4][8][kRedPitch];    // per warp: eight values of its 32 lanes
+    unsigned places;                                      // of grad, taken in this round
+    unsigned maxlast;
+};
+
+// A warp owns an 8x8 block as in the forward; its quarter q the block's columns 2q, 2q + 1 (lane & 7 is
+// the row), so that the sum over a splat's pixels -- rows by shuffles within the quarter, then the
+// quarters as (0 + 2) + (1 + 3), then the warps in order -- runs in a fixed order whichever quarters a
+// splat reaches.
 template <int TW, int TH>
 __global__ void __launch_bounds__(TW * TH / 2) blend_backward_kernel(BackwardIn in, float* __restrict__ grad_pair) {
     chain_entry();
     constexpr int kThreads = TW * TH / 2;
     constexpr int kWarps = kThreads / 32;
     constexpr int kWarpsX = TW / 8;
-    __shared__ float4 s_r0[kBatch];
-    __shared__ float4 s_r1[kBatch];
-    __shared__ float s_b[kBatch];
-    __shared__ unsigned s_pos[kBatch];
-    __shared__ unsigned char s_mask[kBatch];
-    __shared__ unsigned s_hit[kBatch];
-    __shared__ float s_grad[kWarps][kBatch][kG];
-    __shared__ unsigned s_maxlast;
+    constexpr int kCells = TW / 2;  // cells per 8-row band of the tile
+    using Shared = BackwardShared<TW, TH>;
+    constexpr unsigned kPlaces = Shared::kPlaces;
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    Shared& sh = *reinterpret_cast<Shared*>(s_raw);
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quarter = lane >> 3;
     const unsigned gtile = blockIdx.x;
     const unsigned v = find_segment(in.tables.tile_base, in.tables.n_views, gtile);
     const ViewInfo& vi = in.views[v];
     const unsigned local = gtile - vi.tile_base;
     const int tx = static_cast<int>(local % vi.cam.tilesX), ty = static_cast<int>(local / vi.cam.tilesX);
     const int ox = tx * TW, oy = ty * TH;
-    const int x0 = ox + (warp % kWarpsX) * 8 + 2 * (lane & 3), y = oy + (warp / kWarpsX) * 8 + (lane >> 2);
+    const int x0 = ox + (warp % kWarpsX) * 8 + 2 * quarter, y = oy + (warp / kWarpsX) * 8 + (lane & 7);
     const int width = vi.cam.width, height = vi.cam.height;
     const float px0 = x0 + 0.5f, py = y + 0.5f;
     const uint2 range = (in.ctrl->flags & kFlagOverflow) ? make_uint2(0, 0) : in.ranges[gtile];
+    const int cell0 = (warp / kWarpsX) * kCells + (warp % kWarpsX) * 4;  // the warp's first cell in a mask
+    const int sumq = lane & 3, sumk = lane >> 2;  // the quarter and value whose eight lanes this lane sums
 
     PixelState2 st;
     st.T = make_float2(1.f, 1.f);
@@ -173,13 +187,24 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_backward_kernel(BackwardIn 
         st.gg.y = vi.grad_img[3 * p + 1];
         st.gb.y = vi.grad_img[3 * p + 2];
     }
-    if (tid == 0) s_maxlast = range.x;
+    if (tid == 0) {
+        sh.maxlast = range.x;
+        sh.r0[kBatch] = make_float4(0.f, 0.f, 0.f, 0.f);
+        sh.r1[kBatch] = make_float4(0.f, -INFINITY, 0.f, 0.f);
+        sh.b[kBatch] = 0.f;
+    }
+    if (tid < kG) sh.grad[kPlaces * kG + tid] = 0.f;
     __syncthreads();
-    const unsigned mylast = max(st.last0, st.last1);
-    const unsigned wlast = __reduce_max_sync(0xFFFFFFFFu, mylast);
-    if (lane == 0) atomicMax(&s_maxlast, wlast);
+    // Past each quarter's last applied splat, and the tile's.
+    unsigned qlast = max(st.last0, st.last1);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) qlast = max(qlast, __shfl_xor_sync(0xFFFFFFFFu, qlast, o));
+    unsigned lasts[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) lasts[q] = __shfl_sync(0xFFFFFFFFu, qlast, 8 * q);
+    if ((lane & 7) == 0) atomicMax(&sh.maxlast, qlast);
     __syncthreads();
-    const unsigned end = s_maxlast;
+    const unsigned end = sh.maxlast;
 
     // Pairs behind every pixel's last applied splat get zero gradient.
     for (unsigned q = end + tid; q < range.y; q += kThreads) {
@@ -197,72 +222,143 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_backward_kernel(BackwardIn 
     for (unsigned top = end; top > range.x;) {
         const unsigned start = top > range.x + kBatch ? top - kBatch : range.x;
         const unsigned cnt = top - start;
-        // Stage the batch [start, top): records, warp masks and each pair's slot in the
+        // Stage the batch [start, top): records, cell masks and each pair's slot in the
         // depth-ordered pair list (the slot of (Gaussian g, tile t) is offs[rank[g]] plus t's
         // row-major index in g's rectangle).
-        for (unsigned slot = tid; slot < cnt; slot += kThreads) {
-            const unsigned g = in.vals[start + slot];
-            const SplatRecord r = in.rec[g];
-            s_r0[slot] = r.r0;
-            s_r1[slot] = r.r1;
-            s_b[slot] = r.r2.x;
-            // The forward's masks (the same function), so the adjoint walks exactly its splats.
-            s_mask[slot] = static_cast<unsigned char>(staged_block_mask<TW, TH, true>(r, ox, oy));
-            s_hit[slot] = 0;
-            const unsigned j = in.rank[g];
-            const unsigned long long rc = in.rect_sorted[j];
-            const unsigned rx0 = rc & 0xFFFFu, ry0 = (rc >> 16) & 0xFFFFu, rx1 = (rc >> 32) & 0xFFFFu;
-            s_pos[slot] = in.offs[j] + (static_cast<unsigned>(ty) - ry0) * (rx1 - rx0 + 1) + (static_cast<unsigned>(tx) - rx0);
+        for (unsigned slot = tid; slot < kBatch; slot += kThreads) {
+            unsigned m = 0;
+            if (slot < cnt) {
+                const unsigned g = in.vals[start + slot];
+                const SplatRecord r = in.rec[g];
+                constexpr float kMax = 3.40282347e38f;  // an infinite colour as the forward blends it
+                sh.r0[slot] = r.r0;
+                sh.r1[slot] = make_float4(r.r1.x, r.r1.y, fminf(r.r1.z, kMax), fminf(r.r1.w, kMax));
+                sh.b[slot] = fminf(r.r2.x, kMax);
+                m = staged_cell_mask<TW, TH, 2, 8>(r, ox, oy);
+                const unsigned j = in.rank[g];
+                const unsigned long long rc = in.rect_sorted[j];
+                const unsigned rx0 = rc & 0xFFFFu, ry0 = (rc >> 16) & 0xFFFFu, rx1 = (rc >> 32) & 0xFFFFu;
+                sh.pos[slot] =
+                    in.offs[j] + (static_cast<unsigned>(ty) - ry0) * (rx1 - rx0 + 1) + (static_cast<unsigned>(tx) - rx0);
+            }
+            sh.mask[slot] = m;
         }
+        if (tid == 0) sh.places = 0;
         __syncthreads();
-        if (start < wlast) {  // some pixel of the warp applied a splat of this batch
-            for (int c = static_cast<int>((cnt - 1) / 32); c >= 0; --c) {
-                const unsigned idx = c * 32 + lane;
-                unsigned bits = __ballot_sync(0xFFFFFFFFu, idx < cnt && ((s_mask[idx] >> warp) & 1u));
-                while (bits) {
-                    const int b = 31 - __clz(bits);
-                    bits &= ~(1u << b);
-                    const unsigned jj = c * 32 + b;
-                    const unsigned pos = start + jj;
-                    if (pos >= wlast) continue;  // behind every pixel's last applied splat
-                    const float4 r0 = s_r0[jj];
-                    const float4 r1 = s_r1[jj];
-                    const float rb = s_b[jj];
-                    const float dy = __fsub_rn(py, r0.y);
-                    float2 dx;
-                    const float2 pp = splat_exponents2(r0, r1, make_float2(px0, px0 + 1.0f), dy, dx);
-                    float2 G[kG];
-                    const bool any = pixel_step2(st, pos, pp, dx, dy, r0, r1, rb, G);
-                    // No pixel of the warp took the splat: its share is zero, leave it out of the sum.
-                    if (!__any_sync(0xFFFFFFFFu, any)) continue;
-                    float g[kG];
+        // The round takes the staged splats from `first` on: as many, from the back, as surely find
+        // places for their sums. Every warp finds the same number.
+        unsigned first = 0;
+        if (kPlaces < kBatch * Shared::kLists) {
+            constexpr int kPer = kBatch / 32;
+            unsigned need[kPer], total = 0;
 #pragma unroll
-                    for (int q = 0; q < kG; ++q) g[q] = any ? G[q].x + G[q].y : 0.f;
-                    int k;
-                    const float sum = warp_reduce9(g, lane, k);
-                    if (k >= 0) s_grad[warp][jj][k] = sum;
-                    if (lane == 0) atomicOr(&s_hit[jj], 1u << warp);
+            for (int k = kPer - 1; k >= 0; --k) {
+                total += __popc(sh.mask[lane * kPer + k]);
+                need[k] = total;
+            }
+            const unsigned behind = __reduce_add_sync(0xFFFFFFFFu, total) - warp_incl_scan(total);
+            unsigned fit = 0;
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) fit += need[k] + behind <= kPlaces;
+            first = kBatch - __reduce_add_sync(0xFFFFFFFFu, fit);
+        }
+        // Each quarter's splats of the round, back to front, and the places of their sums.
+        unsigned n[4] = {0, 0, 0, 0};
+        unsigned base = 0;
+        {
+            unsigned bits[4][kBatch / 32];
+#pragma unroll
+            for (int c = kBatch / 32 - 1; c >= 0; --c) {
+                const unsigned idx = c * 32 + lane;
+                const unsigned m = idx >= first && idx < cnt ? sh.mask[idx] >> cell0 : 0u;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    bits[q][c] = __ballot_sync(0xFFFFFFFFu, ((m >> q) & 1u) && start + idx < lasts[q]);
+                    n[q] += __popc(bits[q][c]);
                 }
             }
+            if (lane == 0) base = atomicAdd(&sh.places, n[0] + n[1] + n[2] + n[3]);
+            base = __shfl_sync(0xFFFFFFFFu, base, 0);
+            unsigned at0[4] = {base, base + n[0], base + n[0] + n[1], base + n[0] + n[1] + n[2]};
+            unsigned seen[4] = {0, 0, 0, 0};
+            const unsigned above = ~(lanemask_lt() | (1u << lane));
+#pragma unroll
+            for (int c = kBatch / 32 - 1; c >= 0; --c) {
+                const unsigned idx = c * 32 + lane;
+                unsigned short at[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const unsigned i = seen[q] + __popc(bits[q][c] & above);
+                    const bool mine = (bits[q][c] >> lane) & 1u;
+                    at[q] = static_cast<unsigned short>((mine ? at0[q] + i : kPlaces) * kG);
+                    if (mine) sh.list[warp * 4 + q][i] = static_cast<unsigned char>(idx);
+                    seen[q] += __popc(bits[q][c]);
+                }
+                *reinterpret_cast<ushort4*>(&sh.at[idx][warp * 4]) = make_ushort4(at[0], at[1], at[2], at[3]);
+            }
+        }
+        const unsigned longest = max(max(n[0], n[1]), max(n[2], n[3]));
+        const unsigned own = quarter == 0 ? n[0] : quarter == 1 ? n[1] : quarter == 2 ? n[2] : n[3];
+        unsigned char* list = sh.list[warp * 4 + quarter];
+        for (unsigned i = own + (lane & 7); i < longest; i += 8) list[i] = kBatch;
+        __syncwarp();
+        const auto place = [&](int q) {  // of the quarter's first sum
+            return base + (q > 0 ? n[0] : 0u) + (q > 1 ? n[1] : 0u) + (q > 2 ? n[2] : 0u);
+        };
+        // This lane writes one of the first eight values of quarter sumq, and the ninth of its own.
+        const unsigned sum_own = sumq == 0 ? n[0] : sumq == 1 ? n[1] : sumq == 2 ? n[2] : n[3];
+        const unsigned last_own = (lane & 7) == 0 ? own : 0u;
+        float* out = sh.grad + place(sumq) * kG + sumk;
+        float* last = sh.grad + place(quarter) * kG + 8;
+        float* red = sh.red[warp][0] + lane;
+        const float4* redq = reinterpret_cast<const float4*>(sh.red[warp][sumk] + 8 * sumq);
+        for (unsigned i = 0; i < longest; ++i, out += kG, last += kG) {
+            const unsigned jj = list[i];
+            const float4 r0 = sh.r0[jj];
+            const float4 r1 = sh.r1[jj];
+            const float rb = sh.b[jj];
+            const float dy = __fsub_rn(py, r0.y);
+            float2 dx;
+            const float2 pp = splat_exponents2(r0, r1, make_float2(px0, px0 + 1.0f), dy, dx);
+            const PixelTest2 test = pixel_test2(st, start + jj, pp, r1.y);
+            float sum = 0.f, ninth = 0.f;
+            if (__any_sync(0xFFFFFFFFu, test.v0 || test.v1)) {  // else the sums are zero
+                float g[kG];
+                pixel_step2(st, test, dx, dy, r0, r1, rb, g);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) red[k * kRedPitch] = g[k];
+                ninth = g[8];
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) ninth += __shfl_xor_sync(0xFFFFFFFFu, ninth, o);
+                __syncwarp();
+                // The eight rows in the order of the shuffles above: 4 apart, 2 apart, neighbours.
+                const float4 lo = redq[0], hi = redq[1];
+                const float2 even = __fadd2_rn(make_float2(lo.x, lo.y), make_float2(hi.x, hi.y));
+                const float2 odd = __fadd2_rn(make_float2(lo.z, lo.w), make_float2(hi.z, hi.w));
+                const float2 both = __fadd2_rn(even, odd);
+                sum = both.x + both.y;
+                __syncwarp();
+            }
+            if (i < sum_own) *out = sum;
+            if (i < last_own) *last = ninth;
         }
         __syncthreads();
-        // Fixed-order sum over the warps; every staged pair's slot is written.
-        for (unsigned slot = tid; slot < cnt; slot += kThreads) {
-            const unsigned hit = s_hit[slot];
-            float acc[kG];
+        // Fixed-order sum over the quarters and warps; every pair of the round is written. Neighbouring
+        // threads take the values of one pair, so that a store covers whole pairs.
+        for (unsigned e = first * kG + tid; e < cnt * kG; e += kThreads) {
+            const unsigned slot = e / kG, k = e - slot * kG;
+            float acc = 0.f;
 #pragma unroll
-            for (int k = 0; k < kG; ++k) acc[k] = 0.f;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w)
-                if (hit & (1u << w))
-#pragma unroll
-                    for (int k = 0; k < kG; ++k) acc[k] += s_grad[w][slot][k];
-            float* out = grad_pair + static_cast<size_t>(s_pos[slot]) * kG;
-#pragma unroll
-            for (int k = 0; k < kG; ++k) out[k] = acc[k];
+            for (int w = 0; w < kWarps; ++w) {
+                const ushort4 at = *reinterpret_cast<const ushort4*>(&sh.at[slot][4 * w]);
+                const float q0 = sh.grad[at.x + k], q1 = sh.grad[at.y + k];
+                const float q2 = sh.grad[at.z + k], q3 = sh.grad[at.w + k];
+                acc += (q0 + q2) + (q1 + q3);
+            }
+            grad_pair[static_cast<size_t>(sh.pos[slot]) * kG + k] = acc;
         }
         __syncthreads();
-        top = start;
+        top = start + first;
     }
 }
 
@@ -633,13 +729,29 @@ __global__ void __launch_bounds__(128, 4) gauss_backward_kernel(const BatchScene
 
 }  // namespace
 
+namespace {
+template <int TW, int TH>
+void launch_blend_backward_t(const BackwardIn& in, unsigned tiles, float* grad_pair, cudaStream_t stream) {
+    constexpr int kDevices = 64;
+    static std::atomic<bool> raised[kDevices];  // the dynamic shared memory limit, once per device
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kDevices && !raised[dev]) {
+        if (cudaFuncSetAttribute(blend_backward_kernel<TW, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(sizeof(BackwardShared<TW, TH>))) == cudaSuccess)
+            raised[dev] = true;
+    }
+    cudaGetLastError();  // a failed raise shows up as the launch's error
+    launch_chained_smem(blend_backward_kernel<TW, TH>, dim3(tiles), dim3(TW * TH / 2), sizeof(BackwardShared<TW, TH>),
+                        stream, in, grad_pair);
+}
+}  // namespace
+
 void launch_blend_backward(const BackwardIn& in, unsigned tiles, int tile_w, int tile_h, float* grad_pair,
                            cudaStream_t stream) {
     if (tiles == 0) return;
-    if (tile_w == 8) launch_chained(blend_backward_kernel<8, 8>, dim3(tiles), dim3(32), stream, in, grad_pair);
-    else if (tile_h == 32)
-        launch_chained(blend_backward_kernel<16, 32>, dim3(tiles), dim3(256), stream, in, grad_pair);
-    else launch_chained(blend_backward_kernel<16, 16>, dim3(tiles), dim3(128), stream, in, grad_pair);
+    if (tile_w == 8) launch_blend_backward_t<8, 8>(in, tiles, grad_pair, stream);
+    else if (tile_h == 32) launch_blend_backward_t<16, 32>(in, tiles, grad_pair, stream);
+    else launch_blend_backward_t<16, 16>(in, tiles, grad_pair, stream);
 }
 
 namespace {

@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_kernel(const uint2* __restr
                 s_r0[slot] = r.r0;
                 s_r1[slot] = make_float4(r.r1.x, r.r1.y, fminf(r.r1.z, kMax), fminf(r.r1.w, kMax));
                 s_b[slot] = fminf(r.r2.x, kMax);
-                m = staged_cell_mask<TW, TH>(r, ox, oy);
+                m = staged_cell_mask<TW, TH, 4, 4>(r, ox, oy);
             }
             s_mask[slot] = m;
         }

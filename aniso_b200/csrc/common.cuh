@@ -274,13 +274,11 @@ __device__ __forceinline__ float ex2_approx(float x) {
 }
 
 // Blend record: three float4 per visible Gaussian.
-//   r0 = (u, v, A2, B2)     r1 = (C2, L, r, g)     r2 = (b, bx, by, block bits)
+//   r0 = (u, v, A2, B2)     r1 = (C2, L, r, g)     r2 = (b, bx, by, 0)
 // where the exponent of the Gaussian in base 2 is A2 dx^2 + B2 dx dy + C2 dy^2 (the conic scaled
 // by -log2(e)/2, -log2(e), -log2(e)/2), L = log2(opacity), and bx / by hold two int16 pixel bounds
 // (lo | hi << 16): the pixels that lie both in the splat's 8x8-tile rectangle (render.cpp:166-171)
-// and inside the ellipse where alpha can reach 1/255 (with a safety margin); the block bits
-// (record_block_bits) mark the 8x8 pixel blocks of those bounds where the splat can pass the
-// alpha test.
+// and inside the bounding box of the ellipse where alpha can reach 1/255 (with a safety margin).
 struct SplatRecord {
     float4 r0, r1, r2;
 };
@@ -322,113 +320,8 @@ __device__ __forceinline__ float sqrt_mufu(float x) {  // MUFU square root, rela
     return y;
 }
 
-// The x-offset interval [xl, xr] (from the splat centre) over which A x^2 + B x y + C y^2 >= D for
-// some y in [Y0, Y1]; false when there is none. The form is concave (A, C < 0, 4AC > B^2), so the
-// region is an ellipse: its right boundary is concave in y, largest (the half-width W) at
-// y = yr = -B W / 2C, so over the band it is largest at the band's point nearest yr (there the
-// larger root of the quadratic in x); the left boundary likewise, mirrored (y = -yr). inv2a =
-// 1 / 2A. MUFU square roots: the caller widens the interval far beyond their error.
-__device__ __forceinline__ bool band_extent(float A, float B, float C, float D, float inv2a, float W, float yr,
-                                            float Y0, float Y1, float& xl, float& xr) {
-    const auto root = [&](float Y, float sign, float& x) {  // sign -1: the larger root, +1: the smaller
-        const float by = B * Y, disc = by * by - 4.f * A * (C * Y * Y - D);
-        if (!(disc >= 0.f)) return false;
-        x = (sign * sqrt_mufu(disc) - by) * inv2a;
-        return true;
-    };
-    if (yr >= Y0 && yr <= Y1) xr = W;
-    else if (!root(yr > Y1 ? Y1 : Y0, -1.f, xr)) return false;
-    const float yl = -yr;
-    if (yl >= Y0 && yl <= Y1) xl = -W;
-    else if (!root(yl > Y1 ? Y1 : Y0, 1.f, xl)) return false;
-    return xl <= xr;
-}
-
-// The block bits of a blend record (its r2.w), made once per visible entry by the training
-// preprocess (the plain one leaves every bit set): over the 8x8 pixel blocks (absolute: block x
-// covers pixels [8x, 8x + 7]) that the splat's pixel bounds (r2.y, r2.z: its 8x8-tile rectangle of
-// the CPU renderer cut by the bounding box of the ellipse where alpha can reach 1/255) overlap,
-// x0b = xlo >> 3 .. and wb blocks wide, bit j * wb + i is set unless the splat's exponent stays
-// below log2(1/255) at every pixel centre of block (x0b + i, y0b + j): per block row, the x-extent
-// of the ellipse over the row band's centre offsets (band_extent, a continuous superset of the
-// centres), widened, against the blocks' centre offsets. The cut is lowered by 0.02 plus a term
-// relative to the size of the form's terms over the bounds (in log2 units), and the extent widened
-// by 1e-3 of the half-width plus 0.01 pixel, which covers the rounding of this test and of the
-// blend's own evaluation. Bounds of more than 32 blocks, or a degenerate form (a coefficient that
-// is 0 or not finite, or not concave), set every bit. A blend skips a splat on a block whose bit is
-// clear: no pixel there could take anything from it, so the image does not change (and does not
-// depend on the tile shape: the blocks are the image's, not the tile's); only warp steps that could
-// apply nothing are saved.
-__device__ __forceinline__ unsigned record_block_bits(const SplatRecord& r) {
-    constexpr float kCut = -7.99435343685885793f;  // log2(1/255)
-    const unsigned bx = __float_as_uint(r.r2.y), by = __float_as_uint(r.r2.z);
-    const int xlo = unpack_lo(bx), xhi = unpack_hi(bx), ylo = unpack_lo(by), yhi = unpack_hi(by);
-    if (xhi < xlo || yhi < ylo) return 0u;
-    const int x0b = xlo >> 3, y0b = ylo >> 3, wb = (xhi >> 3) - x0b + 1, hb = (yhi >> 3) - y0b + 1;
-    const float u = r.r0.x, v = r.r0.y, A = r.r0.z, B = r.r0.w, C = r.r1.x, L = r.r1.y;
-    const float det4 = 4.f * A * C - B * B;
-    if (wb * hb > 32 || !(A < 0.f && C < 0.f && det4 > 0.f && isfinite(A + B + C + L + det4))) return 0xFFFFFFFFu;
-    const float mx = fmaxf(fabsf(xlo + 0.5f - u), fabsf(xhi + 0.5f - u));
-    const float my = fmaxf(fabsf(ylo + 0.5f - v), fabsf(yhi + 0.5f - v));
-    const float size = fabsf(A) * mx * mx + fabsf(B) * mx * my + fabsf(C) * my * my;
-    const float D = kCut - 0.02f - 1e-5f * size - L;  // the form must reach D somewhere
-    if (D > 0.f) return 0u;                             // it cannot: its largest value is 0
-    const float W = sqrt_mufu(D * (4.f * C) * __frcp_rn(det4));  // half-width: D / (A - B^2 / 4C)
-    const float yr = -B * W * __frcp_rn(2.f * C);
-    const float inv2a = __frcp_rn(2.f * A);
-    const float eps = 1e-3f * W + 0.01f;
-    unsigned bits = 0;
-    for (int j = 0; j < hb; ++j) {
-        const int y0 = max(ylo, 8 * (y0b + j)), y1 = min(yhi, 8 * (y0b + j) + 7);
-        float xl, xr;
-        if (!band_extent(A, B, C, D, inv2a, W, yr, y0 + 0.5f - v, y1 + 0.5f - v, xl, xr)) continue;
-        // blocks whose centre offsets [8 b + 0.5 - u, 8 b + 7.5 - u] meet [xl - eps, xr + eps]
-        const int lo = max(0, static_cast<int>(ceilf((u + xl - eps - 7.5f) * 0.125f)) - x0b);
-        const int hi = min(wb - 1, static_cast<int>(floorf((u + xr + eps - 0.5f) * 0.125f)) - x0b);
-        if (lo <= hi) bits |= ((2u << hi) - (1u << lo)) << (j * wb);  // bits lo..hi (2u << 31 wraps to 0)
-    }
-    return bits;
-}
-
-// The 8x8 pixel blocks of a TW x TH tile at pixel (ox, oy, multiples of 8) that a staged splat
-// record may touch, bit rr * (TW / 8) + c for block (c, rr): the blocks its pixel bounds overlap,
-// and with kBits only those whose bit in the record's block bits is set. The training forward and
-// the adjoint stage the same masks.
-template <int TW, int TH, bool kBits>
-__device__ __forceinline__ unsigned staged_block_mask(const SplatRecord& r, int ox, int oy) {
-    constexpr int kWX = TW / 8, kWY = TH / 8;
-    const unsigned bx = __float_as_uint(r.r2.y), by = __float_as_uint(r.r2.z);
-    const int xlo = unpack_lo(bx), xhi = unpack_hi(bx), ylo = unpack_lo(by), yhi = unpack_hi(by);
-    unsigned m = 0;
-    if (!kBits) {
-        unsigned cols = 0;
-#pragma unroll
-        for (int c = 0; c < kWX; ++c)
-            if (xlo <= ox + 8 * c + 7 && xhi >= ox + 8 * c) cols |= 1u << c;
-#pragma unroll
-        for (int rr = 0; rr < kWY; ++rr)
-            if (ylo <= oy + 8 * rr + 7 && yhi >= oy + 8 * rr) m |= cols << (kWX * rr);
-        return m;
-    }
-    const unsigned bits = __float_as_uint(r.r2.w);
-    const int x0b = xlo >> 3, y0b = ylo >> 3, wb = (xhi >> 3) - x0b + 1;
-#pragma unroll
-    for (int rr = 0; rr < kWY; ++rr) {
-        const int py = oy + 8 * rr;
-        if (ylo > py + 7 || yhi < py) continue;
-#pragma unroll
-        for (int c = 0; c < kWX; ++c) {
-            const int px = ox + 8 * c;
-            if (xlo > px + 7 || xhi < px) continue;
-            const int idx = ((py >> 3) - y0b) * wb + ((px >> 3) - x0b);
-            if (idx >= 32 || ((bits >> idx) & 1u)) m |= 1u << (rr * kWX + c);
-        }
-    }
-    return m;
-}
-
-// The 4x4-pixel cells of a TW x TH tile at pixel (ox, oy, multiples of 8) that a staged splat record
-// may touch, bit rr * (TW / 4) + c for cell (c, rr): the cells its pixel bounds overlap, less those
+// The CW x CH-pixel cells of a TW x TH tile at pixel (ox, oy, multiples of 8) that a staged splat record
+// may touch, bit rr * (TW / CW) + c for cell (c, rr): the cells its pixel bounds overlap, less those
 // where its exponent stays below log2(1/255) at every pixel centre (no pixel there could take
 // anything from it, so leaving them out changes no result and the image does not depend on the tile
 // shape). The test, per row of cells, is on the x-extent of the ellipse where the exponent reaches
@@ -443,20 +336,20 @@ __device__ __forceinline__ unsigned staged_block_mask(const SplatRecord& r, int 
 // for needles, whose terms cancel), and the extent is widened by 1e-3 of the half-width plus 0.01
 // pixel (MUFU square roots and reciprocals, relative error ~2^-22). A degenerate form (a coefficient
 // that is 0 or not finite, or not concave) keeps every cell of the bounds.
-template <int TW, int TH>
+template <int TW, int TH, int CW, int CH>
 __device__ __forceinline__ unsigned staged_cell_mask(const SplatRecord& r, int ox, int oy) {
     constexpr float kCut = -7.99435343685885793f;  // log2(1/255)
-    constexpr int kC = TW / 4, kR = TH / 4;
+    constexpr int kC = TW / CW, kR = TH / CH;
     static_assert(kC * kR <= 32, "one bit per cell");
     const unsigned bx = __float_as_uint(r.r2.y), by = __float_as_uint(r.r2.z);
     const int xlo = unpack_lo(bx), xhi = unpack_hi(bx), ylo = unpack_lo(by), yhi = unpack_hi(by);
     unsigned cols = 0, m = 0;
 #pragma unroll
     for (int c = 0; c < kC; ++c)
-        if (xlo <= ox + 4 * c + 3 && xhi >= ox + 4 * c) cols |= 1u << c;
+        if (xlo <= ox + CW * c + CW - 1 && xhi >= ox + CW * c) cols |= 1u << c;
 #pragma unroll
     for (int rr = 0; rr < kR; ++rr)
-        if (ylo <= oy + 4 * rr + 3 && yhi >= oy + 4 * rr) m |= cols << (kC * rr);
+        if (ylo <= oy + CH * rr + CH - 1 && yhi >= oy + CH * rr) m |= cols << (kC * rr);
 
     const float u = r.r0.x, v = r.r0.y, A = r.r0.z, B = r.r0.w, C = r.r1.x, L = r.r1.y;
     const float det4 = 4.f * A * C - B * B;
@@ -474,14 +367,14 @@ __device__ __forceinline__ unsigned staged_cell_mask(const SplatRecord& r, int o
     unsigned keep = 0;
 #pragma unroll
     for (int rr = 0; rr < kR; ++rr) {
-        const float Y0 = static_cast<float>(oy + 4 * rr) + 0.5f - v, Y1 = Y0 + 3.f;
+        const float Y0 = static_cast<float>(oy + CH * rr) + 0.5f - v, Y1 = Y0 + (CH - 1);
         const float ya = fminf(fmaxf(yr, Y0), Y1), yb = fminf(fmaxf(-yr, Y0), Y1);
         const float da = fmaf(-det4 * ya, ya, ad4), db = fmaf(-det4 * yb, yb, ad4);
         const float xr = (-sqrt_mufu(fmaxf(da, 0.f)) - B * ya) * inv2a;
         const float xl = (sqrt_mufu(fmaxf(db, 0.f)) - B * yb) * inv2a;
-        // cells whose centre offsets [4 c + 0.5, 4 c + 3.5] (from ox) meet [xl - eps, xr + eps]
-        const int lo = max(0, __float2int_ru((centre + xl - eps - 3.5f) * 0.25f));
-        const int hi = min(kC - 1, __float2int_rd((centre + xr + eps - 0.5f) * 0.25f));
+        // cells whose centre offsets [CW c + 0.5, CW (c + 1) - 0.5] (from ox) meet [xl - eps, xr + eps]
+        const int lo = max(0, __float2int_ru((centre + xl - eps - (CW - 0.5f)) * (1.0f / CW)));
+        const int hi = min(kC - 1, __float2int_rd((centre + xr + eps - 0.5f) * (1.0f / CW)));
         if (da >= 0.f && db >= 0.f && lo <= hi) keep |= ((2u << hi) - (1u << lo)) << (kC * rr);
     }
     return m & keep;

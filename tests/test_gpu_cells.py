@@ -57,3 +57,29 @@ def test_no_pixel_loses_a_splat(tile):
         assert (img[..., 0][clear] >= low[clear]).all(), (k, tile)
         checked += int(clear.sum())
     assert checked > 20_000
+
+
+@pytest.mark.parametrize("tile", [(16, 16), (16, 32)])
+def test_adjoint_rounds_are_cut_where_their_sums_run_out_of_room(tile):
+    """Splats that each touch every cell of a tile: a round of 128 of them needs four times the places
+    the 16x16 and 16x32 tiles have, so rounds are cut; an 8x8 tile has room for all of its round."""
+    import torch
+
+    from aniso_b200 import scenes
+    from aniso_b200.autograd import rasterize_batch
+
+    raw = scenes.make_raw_scene(700, (-1.0, -0.8, 2.0), (1.0, 0.8, 4.0), seed=5)
+    n = raw.n
+    sh = np.concatenate([raw.f_dc.reshape(n, 1, 3), raw.f_rest.reshape(n, 3, 15).transpose(0, 2, 1)], 1)
+    arrays = [raw.xyz, raw.scale + np.float32(3.5), raw.rot, raw.opacity - np.float32(3.0), np.ascontiguousarray(sh)]
+    cam = scenes.Camera(75, 61, 70.0, 70.0, 37.5, 30.5, np.eye(3), np.zeros(3))
+    up = torch.randn(cam.height, cam.width, 3, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+    got = {}
+    for shape in (tile, (8, 8)):
+        leaves = [torch.tensor(a, dtype=torch.float32, device="cuda", requires_grad=True) for a in arrays]
+        (img,) = rasterize_batch([leaves], [cam], [0], tile=shape, use_graph=False)
+        got[shape] = [img.detach()] + list(torch.autograd.grad(img, leaves, up))
+    assert torch.equal(got[tile][0], got[(8, 8)][0])
+    # The same terms summed per tile of another grid: fp32 sums of up to 4575 pixels, 1e-5 norm-wise.
+    for a, b in zip(got[tile][1:], got[(8, 8)][1:]):
+        assert float((a.double() - b.double()).norm()) <= 1e-5 * float(b.double().norm())
