@@ -209,8 +209,8 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_backward_kernel(BackwardIn 
     // Pairs behind every pixel's last applied splat get zero gradient.
     for (unsigned q = end + tid; q < range.y; q += kThreads) {
         const unsigned g = in.vals[q];
-        const unsigned j = in.rank[g];
-        const unsigned long long rc = in.rect_sorted[j];
+        const unsigned j = in.rank ? in.rank[g] : g;
+        const unsigned long long rc = in.rect[j];
         const unsigned rx0 = rc & 0xFFFFu, ry0 = (rc >> 16) & 0xFFFFu, rx1 = (rc >> 32) & 0xFFFFu;
         float* out = grad_pair +
                      static_cast<size_t>(in.offs[j] + (static_cast<unsigned>(ty) - ry0) * (rx1 - rx0 + 1) +
@@ -222,9 +222,8 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_backward_kernel(BackwardIn 
     for (unsigned top = end; top > range.x;) {
         const unsigned start = top > range.x + kBatch ? top - kBatch : range.x;
         const unsigned cnt = top - start;
-        // Stage the batch [start, top): records, cell masks and each pair's slot in the
-        // depth-ordered pair list (the slot of (Gaussian g, tile t) is offs[rank[g]] plus t's
-        // row-major index in g's rectangle).
+        // Stage the batch [start, top): records, cell masks and each pair's gradient slot (the slot of
+        // (entry g, tile t) is g's first one plus t's row-major index in g's rectangle).
         for (unsigned slot = tid; slot < kBatch; slot += kThreads) {
             unsigned m = 0;
             if (slot < cnt) {
@@ -235,8 +234,8 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_backward_kernel(BackwardIn 
                 sh.r1[slot] = make_float4(r.r1.x, r.r1.y, fminf(r.r1.z, kMax), fminf(r.r1.w, kMax));
                 sh.b[slot] = fminf(r.r2.x, kMax);
                 m = staged_cell_mask<TW, TH, 2, 8>(r, ox, oy);
-                const unsigned j = in.rank[g];
-                const unsigned long long rc = in.rect_sorted[j];
+                const unsigned j = in.rank ? in.rank[g] : g;
+                const unsigned long long rc = in.rect[j];
                 const unsigned rx0 = rc & 0xFFFFu, ry0 = (rc >> 16) & 0xFFFFu, rx1 = (rc >> 32) & 0xFFFFu;
                 sh.pos[slot] =
                     in.offs[j] + (static_cast<unsigned>(ty) - ry0) * (rx1 - rx0 + 1) + (static_cast<unsigned>(tx) - rx0);
@@ -452,6 +451,14 @@ __device__ __forceinline__ void copy_words(T& dst, const T& src) {
         reinterpret_cast<unsigned*>(&dst)[threadIdx.x] = reinterpret_cast<const unsigned*>(&src)[threadIdx.x];
 }
 
+// Tiles per row of a rectangle, and its tiles (none where it is empty: 1 .. 0).
+__device__ __forceinline__ unsigned rect_width(unsigned long long r) {
+    return static_cast<unsigned>((r >> 32) & 0xFFFFu) - static_cast<unsigned>(r & 0xFFFFu) + 1u;
+}
+__device__ __forceinline__ unsigned rect_tiles(unsigned long long r) {
+    return rect_width(r) * (static_cast<unsigned>(r >> 48) - static_cast<unsigned>((r >> 16) & 0xFFFFu) + 1u);
+}
+
 // Held to 128 registers (four CTAs per SM): the kernel waits on memory, and the extra warps
 // measured faster where it runs many times per step (the 8-scene training batch: 27.0 -> 25.2 ms a
 // step; 102 registers spilled and was no faster; the adjoint blend held to 64 was slower).
@@ -463,7 +470,8 @@ __global__ void __launch_bounds__(128, 4) gauss_backward_kernel(const BatchScene
                                                              const unsigned* __restrict__ list_count,
                                                              const unsigned* __restrict__ rank,
                                                              const unsigned* __restrict__ offs,
-                                                             const unsigned long long* __restrict__ rect_sorted,
+                                                             const unsigned long long* __restrict__ rect,
+                                                             const unsigned long long* __restrict__ whole,
                                                              const float* __restrict__ grad_pair) {
     chain_entry();
     __shared__ CamParams s_cam;
@@ -492,33 +500,46 @@ __global__ void __launch_bounds__(128, 4) gauss_backward_kernel(const BatchScene
     const bool active = t < count;
     const unsigned e = active ? entry_base + list[t] : entry_base;
     const int64_t i = e - entry_base;
-    unsigned cnt = 0, off = 0;
+    // The slots are those of the (cut) rectangle; `whole` (NULL: the same) is the rectangle before the cut.
+    unsigned cnt = 0, off = 0, cut = 0;
+    unsigned long long rc = 0, wr = 0;
     if (active) {
-        const unsigned j = rank[e];
-        const unsigned long long rc = rect_sorted[j];
-        cnt = ((rc >> 32 & 0xFFFFu) - (rc & 0xFFFFu) + 1) * ((rc >> 48) - (rc >> 16 & 0xFFFFu) + 1);
+        const unsigned j = rank ? rank[e] : e;
+        rc = rect[j];
+        wr = whole ? whole[j] : rc;
+        cut = rect_tiles(rc);
+        cnt = rect_tiles(wr);
         off = offs[j];
     }
     // The sum of the Gaussian's per-pair gradients, in a fixed order: a short list by its own lane,
     // slot after slot; a long one (the nearest splats own thousands of tiles) by the whole warp,
-    // lane l taking slots l, l + 32, ..., then a fixed shuffle tree -- so one huge splat does not
-    // hold its warp for thousands of serial loads.
+    // lane l taking tiles l, l + 32, ... of the whole rectangle, then a fixed shuffle tree -- so one
+    // huge splat does not hold its warp for thousands of serial loads, and a cut rectangle's sum has the
+    // bits of the whole one's (whose other tiles add zeros).
     constexpr unsigned kSolo = 16;
     float g9[kG] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (cnt <= kSolo) {
         const float* gp = grad_pair + static_cast<size_t>(off) * kG;
-        for (unsigned k = 0; k < cnt; ++k)
+        for (unsigned k = 0; k < cut; ++k)
 #pragma unroll
             for (int c = 0; c < kG; ++c) g9[c] += gp[k * kG + c];
     }
     for (unsigned big = __ballot_sync(0xFFFFFFFFu, cnt > kSolo); big; big &= big - 1) {
         const int src = __ffs(big) - 1;
         const unsigned bc = __shfl_sync(0xFFFFFFFFu, cnt, src), bo = __shfl_sync(0xFFFFFFFFu, off, src);
+        const unsigned long long br = __shfl_sync(0xFFFFFFFFu, rc, src), bw = __shfl_sync(0xFFFFFFFFu, wr, src);
+        const unsigned ww = rect_width(bw), cw = rect_width(br), ch = rect_tiles(br) / max(cw, 1u);
+        // The cut rectangle's corner within the whole one (an empty one holds no tile).
+        const unsigned dx = (br & 0xFFFFu) - (bw & 0xFFFFu), dy = (br >> 16 & 0xFFFFu) - (bw >> 16 & 0xFFFFu);
         const float* gp = grad_pair + static_cast<size_t>(bo) * kG;
         float part[kG] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (unsigned k = lane; k < bc; k += 32)
+        for (unsigned k = lane; k < bc; k += 32) {
+            const unsigned row = k / ww, y = row - dy, x = k - row * ww - dx;
+            if (x >= cw || y >= ch) continue;
+            const float* slot = gp + static_cast<size_t>(y * cw + x) * kG;
 #pragma unroll
-            for (int c = 0; c < kG; ++c) part[c] += gp[k * kG + c];
+            for (int c = 0; c < kG; ++c) part[c] += slot[c];
+        }
 #pragma unroll
         for (int c = 0; c < kG; ++c) {
 #pragma unroll
@@ -760,34 +781,39 @@ namespace {
 template <bool kFresh>
 void launch_gauss_backward_t(const GaussBackwardArgs& a, const Ctrl* ctrl, const unsigned* list,
                              const unsigned* list_count, const unsigned* rank, const unsigned* offs,
-                             const unsigned long long* rect_sorted, const float* grad_pair, dim3 grid, dim3 block,
+                             const unsigned long long* rect, const unsigned long long* whole, const float* grad_pair,
+                             dim3 grid, dim3 block,
                              cudaStream_t stream) {
     switch (a.sh_degree) {
         case 0: launch_chained(gauss_backward_kernel<0, kFresh>, grid, block, stream, a.scenes, a.scene, a.views,
-                               a.view, a.grads, ctrl, list, list_count, rank, offs, rect_sorted, grad_pair); break;
+                               a.view, a.grads, ctrl, list, list_count, rank, offs, rect, whole,
+                               grad_pair); break;
         case 1: launch_chained(gauss_backward_kernel<1, kFresh>, grid, block, stream, a.scenes, a.scene, a.views,
-                               a.view, a.grads, ctrl, list, list_count, rank, offs, rect_sorted, grad_pair); break;
+                               a.view, a.grads, ctrl, list, list_count, rank, offs, rect, whole,
+                               grad_pair); break;
         case 2: launch_chained(gauss_backward_kernel<2, kFresh>, grid, block, stream, a.scenes, a.scene, a.views,
-                               a.view, a.grads, ctrl, list, list_count, rank, offs, rect_sorted, grad_pair); break;
+                               a.view, a.grads, ctrl, list, list_count, rank, offs, rect, whole,
+                               grad_pair); break;
         default: launch_chained(gauss_backward_kernel<3, kFresh>, grid, block, stream, a.scenes, a.scene, a.views,
-                                a.view, a.grads, ctrl, list, list_count, rank, offs, rect_sorted, grad_pair); break;
+                                a.view, a.grads, ctrl, list, list_count, rank, offs, rect, whole,
+                               grad_pair); break;
     }
 }
 }  // namespace
 
 void launch_gauss_backward(const GaussBackwardArgs& a, const Ctrl* ctrl, const unsigned* depth_key,
-                           const unsigned* rank, const unsigned* offs, const unsigned long long* rect_sorted,
-                           const float* grad_pair, unsigned* list, unsigned* list_count, cudaStream_t stream) {
+                           const unsigned* rank, const unsigned* offs, const unsigned long long* rect,
+                           const unsigned long long* whole, const float* grad_pair, unsigned* list, unsigned* list_count, cudaStream_t stream) {
     const unsigned lblocks = static_cast<unsigned>((a.n + 256 * kListItems - 1) / (256 * kListItems));
     if (lblocks == 0) return;
     launch_chained(visible_list_kernel, dim3(lblocks), dim3(256), stream, a.n, a.entry_base, depth_key, list,
                    list_count);
     const dim3 grid(static_cast<unsigned>((a.n + 127) / 128)), block(128);
     if (a.fresh)
-        launch_gauss_backward_t<true>(a, ctrl, list, list_count, rank, offs, rect_sorted, grad_pair, grid, block,
+        launch_gauss_backward_t<true>(a, ctrl, list, list_count, rank, offs, rect, whole, grad_pair, grid, block,
                                       stream);
     else
-        launch_gauss_backward_t<false>(a, ctrl, list, list_count, rank, offs, rect_sorted, grad_pair, grid, block,
+        launch_gauss_backward_t<false>(a, ctrl, list, list_count, rank, offs, rect, whole, grad_pair, grid, block,
                                        stream);
 }
 

@@ -2,9 +2,9 @@
 //
 // Everything renders through one plan: V views of S scenes. A frame is a fixed, host-sync-free
 // sequence of kernels on one stream (capturable in a CUDA graph), launched with programmatic
-// stream serialisation: upload of the plan's view table, frame_begin (control block, first digit
-// counts, tile ranges), preprocess, 4 depth LSD passes, pair scan, pair expansion, 1-4 tile LSD
-// passes, tile ranges, blend. After a synchronous frame one more kernel hands the control block
+// stream serialisation: the frame's start (upload of the plan's view table, clears of the control block
+// and the counts), preprocess, the sort (tile ranges, pair scatter, per-tile sort and merge; in small
+// frames the LSD chain: depth passes, pair scan, pair expansion, tile passes or binning), blend. After a synchronous frame one more kernel hands the control block
 // to the host. Data-dependent sizes (visible entries, pairs) stay on the
 // device; grids are sized for capacity and surplus blocks exit at once. The reference instead reads
 // the pair count back mid-frame (gpu_render.cu:329) to size its buffers; here a frame whose pairs
@@ -91,19 +91,37 @@ int bits_for(uint32_t v) {  // bits needed to hold v
 constexpr uint64_t kMaxEntries = 0xFFFFFFFFull;  // entry and tile indices are 32-bit
 constexpr uint64_t kMaxPairs = 0x3FFFFFFFull;    // pair positions and the span arithmetic are 32-bit
 
-// Work buffers of one frame at a time, sized for `n` entries and a pair capacity.
+// The frames the tile sort (sort_tiles.cu) takes: those of at least kTileSortEntries entries (and of at
+// most kTileSortTiles tiles: its counters take 64 bytes a tile). Smaller frames keep the LSD chain: their
+// launch sequence is fixed, kernel by kernel, by the tests. That is not where the two break even:
+// a 5000-Gaussian 640x360 frame takes 61 us with the chain and 27 us with the tile sort, one of 500 57 and
+// 31 us.
+constexpr uint64_t kTileSortEntries = 8192;
+constexpr uint64_t kTileSortTiles = 1ull << 24;
+
+// Work buffers of one frame at a time, sized for `n` entries and a pair capacity. Each sort's own
+// buffers are made when a frame first takes it (prepare).
 struct Arena {
     int64_t n = -1;
     unsigned pair_cap = 0;
     DevBuf<SplatRecord> rec;
     DevBuf<unsigned long long> rect16;
     DevBuf<unsigned> depth_key;
-    DevBuf<unsigned> vis_key[2], vis_idx[2];
-    DevBuf<unsigned> pair_key[2], pair_val[2];
-    DevBuf<unsigned> offs, rank, chunk_start;
-    DevBuf<unsigned long long> rect_sorted;
+    DevBuf<unsigned> pair_val[2];  // sorted entries: of the tile sort in [0], of the LSD chain in either
+    DevBuf<unsigned> offs;
     DevBuf<uint2> ranges;
     DevBuf<Ctrl> ctrl;
+    // The tile sort: the pairs (depth key, entry) being sorted, a copy for lists beyond one merge step,
+    // the tiles' counters, and the chunks of long lists.
+    DevBuf<unsigned long long> pairs, merged;
+    DevBuf<unsigned long long> whole;  // training: the rectangles before they are cut (TileCounts)
+    DevBuf<unsigned> tile_counts, tile_cursor, tile_sums;
+    DevBuf<uint2> chunks;
+    // The LSD chain.
+    DevBuf<unsigned> vis_key[2], vis_idx[2];
+    DevBuf<unsigned> pair_key[2];
+    DevBuf<unsigned> rank, chunk_start;
+    DevBuf<unsigned long long> rect_sorted;
     DevBuf<unsigned> sort_scratch;          // per-span digit counts of the pass in flight
     DevBuf<unsigned long long> span_sum;    // pairs per span of the pair-offset scan
     // The persistent sort (one CTA per SM, `ctas` of them; 0 = the multi-kernel sort runs): two
@@ -125,6 +143,12 @@ struct Arena {
         return ++g;
     }
 
+    template <typename T>
+    int grow(DevBuf<T>& buf, size_t count) {
+        if (count > buf.cap || !buf.p) gen = next_gen();
+        return buf.reserve(count);
+    }
+
     int init(int64_t count, unsigned cap) {
         n = count;
         gen = next_gen();
@@ -132,22 +156,52 @@ struct Arena {
         AB_TRY(rec.reserve(nn));
         AB_TRY(rect16.reserve(nn));
         AB_TRY(depth_key.reserve(nn));
-        for (int k = 0; k < 2; ++k) {
-            AB_TRY(vis_key[k].reserve(nn));
-            AB_TRY(vis_idx[k].reserve(nn));
-        }
-        AB_TRY(ctrl.reserve(1, true));
-        AB_TRY(sort_scratch.reserve(2 * sort_scratch_words()));  // two count matrices and the totals
-        ctas = persistent_sort_ctas();
-        AB_TRY(span_sum.reserve(std::max<size_t>(sort_span_sums(), ctas)));
-        if (ctas) {
-            AB_TRY(pcounts.reserve(2 * persistent_sort_count_words(ctas)));
-            AB_TRY(chunk_first.reserve(ctas + 1));
-        }
         AB_TRY(offs.reserve(nn));
-        AB_TRY(rank.reserve(nn));
-        AB_TRY(rect_sorted.reserve(nn));
-        return grow_pairs(cap);
+        AB_TRY(ctrl.reserve(1, true));
+        ctas = persistent_sort_ctas();
+        pair_cap = cap;
+        return 0;
+    }
+
+    // Whether the tile sort takes a frame (its counters take 64 bytes a tile).
+    bool tile_sorted(uint64_t entries, uint64_t tiles) const {
+        return !ctas && entries >= kTileSortEntries && tiles <= kTileSortTiles;
+    }
+
+    // Everything a frame of `entries` entries and `tiles` tiles needs beyond init (no list of a tile
+    // longer than `longest`): nothing is allocated while the frame is enqueued or captured after this.
+    int prepare(uint64_t entries, uint64_t tiles, uint64_t longest, bool train) {
+        AB_TRY(grow(ranges, static_cast<size_t>(tiles)));
+        AB_TRY(grow(pair_val[0], pair_cap));
+        if (tile_sorted(entries, tiles)) {
+            AB_TRY(grow(pairs, pair_cap));
+            if (train) AB_TRY(grow(whole, static_cast<size_t>(std::max<int64_t>(n, 1))));
+            if (longest > static_cast<uint64_t>(kTileGroup) * kTileChunk) AB_TRY(grow(merged, pair_cap));
+            AB_TRY(grow(tile_counts, tile_count_words(tiles)));
+            AB_TRY(grow(tile_cursor, tile_count_words(tiles)));
+            AB_TRY(grow(tile_sums, tile_sum_words(tiles)));
+            return grow(chunks, tile_chunk_entries(pair_cap));
+        }
+        const size_t nn = static_cast<size_t>(std::max<int64_t>(n, 1));
+        AB_TRY(grow(pair_val[1], pair_cap));
+        for (int k = 0; k < 2; ++k) {
+            AB_TRY(grow(vis_key[k], nn));
+            AB_TRY(grow(vis_idx[k], nn));
+            AB_TRY(grow(pair_key[k], pair_cap));
+        }
+        AB_TRY(grow(rank, nn));
+        AB_TRY(grow(rect_sorted, nn));
+        AB_TRY(grow(chunk_start, chunks_of(pair_cap, expand_chunk_pairs()) + 2));
+        AB_TRY(grow(sort_scratch, 2 * sort_scratch_words()));  // two count matrices and the totals
+        AB_TRY(grow(span_sum, std::max<size_t>(sort_span_sums(), ctas)));
+        if (ctas) {
+            AB_TRY(grow(pcounts, 2 * persistent_sort_count_words(ctas)));
+            return grow(chunk_first, ctas + 1);
+        }
+        if (tiles > bin_tiles && tiles <= bin_max_tiles()) bin_tiles = static_cast<unsigned>(tiles);
+        if (!bin_tiles || pair_cap > bin_max_pairs()) return 0;
+        AB_TRY(grow(bin_counts, bin_count_words(pair_cap, bin_tiles)));
+        return grow(tile_start, bin_max_tiles());
     }
 
     // Makes room for at least `entries` entries (re-initialising when it grows).
@@ -160,41 +214,15 @@ struct Arena {
         return init(entries, static_cast<unsigned>(std::min<uint64_t>(cap, kMaxPairs)));
     }
 
-    // Tile ranges for `tiles` tiles, and the tile binning's buffers when it takes such frames.
-    int reserve_ranges(size_t tiles) {
-        if (tiles > ranges.cap || !ranges.p) gen = next_gen();
-        AB_TRY(ranges.reserve(tiles));
-        if (tiles > bin_tiles && tiles <= bin_max_tiles()) {
-            bin_tiles = static_cast<unsigned>(tiles);
-            return reserve_bins();
-        }
-        return 0;
-    }
-
-    int reserve_bins() {
-        if (!bin_tiles || pair_cap > bin_max_pairs()) return 0;
-        const size_t words = bin_count_words(pair_cap, bin_tiles);
-        if (words > bin_counts.cap || !bin_counts.p || !tile_start.p) gen = next_gen();
-        AB_TRY(bin_counts.reserve(words));
-        return tile_start.reserve(bin_max_tiles());
-    }
-
     // The tile binning can sort a frame of `tiles` tiles at the current pair capacity.
     bool bins_for(unsigned tiles) const {
         return tiles > 0 && tiles <= bin_tiles && pair_cap <= bin_max_pairs() && tile_start.p &&
                bin_counts.cap >= bin_count_words(pair_cap, tiles);
     }
 
-    int grow_pairs(unsigned cap) {
-        if (cap <= pair_cap && pair_key[0].p) return 0;
-        gen = next_gen();
-        for (int k = 0; k < 2; ++k) {
-            AB_TRY(pair_key[k].reserve(cap));
-            AB_TRY(pair_val[k].reserve(cap));
-        }
-        pair_cap = cap;
-        AB_TRY(reserve_bins());
-        return chunk_start.reserve(chunks_of(cap, expand_chunk_pairs()) + 2);
+    // A larger pair capacity, from the next prepare on (which replaces the pair buffers).
+    void grow_pairs(unsigned cap) {
+        if (cap > pair_cap) pair_cap = cap;
     }
 };
 
@@ -271,6 +299,32 @@ int enqueue_sort_persistent(Arena& A, unsigned entries, unsigned tiles, const Ba
     AB_CUDA(launch_sort_frame(a, A.ctas, st));
     *final_buf = a.tile_passes & 1;
     return 0;
+}
+
+// The sort of a frame that the tile sort takes; the sorted entries are in pair_val[0]. keep_slots: also
+// each visible entry's first gradient slot, in A.offs.
+void enqueue_tile_sort(Arena& A, unsigned entries, unsigned longest, unsigned tiles, const BatchTables& tables,
+                       bool keep_slots, cudaStream_t st) {
+    TileSortArgs a{};
+    a.depth_key = A.depth_key.p;
+    a.rect16 = A.rect16.p;
+    a.entries = entries;
+    a.longest = longest;
+    a.tables = tables;
+    a.tiles = tiles;
+    a.counts = A.tile_counts.p;
+    a.cursor = A.tile_cursor.p;
+    a.sums = A.tile_sums.p;
+    a.ranges = A.ranges.p;
+    a.chunks = A.chunks.p;
+    a.chunk_cap = static_cast<unsigned>(tile_chunk_entries(A.pair_cap));
+    a.pairs = A.pairs.p;
+    a.merged = A.merged.p;
+    a.vals = A.pair_val[0].p;
+    a.offs = keep_slots ? A.offs.p : nullptr;
+    a.capacity = A.pair_cap;
+    a.ctrl = A.ctrl.p;
+    launch_tile_sort(a, st);
 }
 
 // Depth passes over `entries` depth keys (the first compacts the visible ones), pair scan and
@@ -501,6 +555,12 @@ struct Plan {
             if (v.scene >= boxes.size() || !boxes[v.scene] || !depth_short(*boxes[v.scene], v.cam)) short_depth = false;
     }
 
+    // The most entries a view has: no tile's list is longer.
+    uint64_t longest() const {
+        uint64_t most = 0;
+        for (const auto& v : views) most = std::max<uint64_t>(most, v.n);
+        return most;
+    }
     // The largest degree any view is coloured with (the preprocess kernel's instantiation).
     int rendered_degree() const {
         int d = 0;
@@ -644,16 +704,18 @@ struct Slot {
 };
 
 void launch_preprocess_any(const BatchScene<SceneView>* sc, const Plan<SceneView>& P, const ViewInfo* views, Arena& A,
-                           const DebugProjection* dbg, const PassCounts& counts, cudaStream_t st) {
+                           const DebugProjection* dbg, const PassCounts& counts, const TileCounts& tile_counts,
+                           cudaStream_t st) {
     launch_preprocess(sc, static_cast<unsigned>(P.scenes.size()), P.pre_blocks, views, P.rendered_degree(),
                       P.shape.tile_w, P.shape.tile_h, A.rec.p, A.rect16.p, A.depth_key.p, dbg, counts,
-                      static_cast<unsigned>(P.entries), st);
+                      static_cast<unsigned>(P.entries), tile_counts, st);
 }
 void launch_preprocess_any(const BatchScene<RawParams>* sc, const Plan<RawParams>& P, const ViewInfo* views,
-                           Arena& A, const DebugProjection*, const PassCounts& counts, cudaStream_t st) {
+                           Arena& A, const DebugProjection*, const PassCounts& counts, const TileCounts& tile_counts,
+                           cudaStream_t st) {
     launch_preprocess_raw(sc, static_cast<unsigned>(P.scenes.size()), P.pre_blocks, views, P.rendered_degree(),
                           P.shape.tile_w, P.shape.tile_h, A.rec.p, A.rect16.p, A.depth_key.p, counts,
-                          static_cast<unsigned>(P.entries), st);
+                          static_cast<unsigned>(P.entries), tile_counts, st);
 }
 
 // Enqueues one frame of a plan. ev (4 events, may be NULL) brackets the stages.
@@ -663,17 +725,29 @@ int enqueue_plan(Arena& A, Slot& slot, const Plan<Src>& P, cudaStream_t st, cuda
     const ViewInfo* views = nullptr;
     const BatchScene<Src>* scenes = nullptr;
     BatchTables tables;
-    AB_TRY(A.reserve_ranges(static_cast<size_t>(P.tiles)));
+    AB_TRY(A.prepare(P.entries, P.tiles, P.longest(), train));
+    const unsigned entries = static_cast<unsigned>(P.entries), tiles = static_cast<unsigned>(P.tiles);
+    const bool by_tile = A.tile_sorted(P.entries, P.tiles);
     unsigned zero_words = 0;
-    const PassCounts first = first_pass_counts(A, static_cast<unsigned>(P.entries), P.short_depth, &zero_words);
+    const PassCounts first = by_tile ? PassCounts{} : first_pass_counts(A, entries, P.short_depth, &zero_words);
+    // A frame that is only sorted shows its pairs, so it keeps the whole rectangles.
+    const bool cut = by_tile && !stop_after_sort;
+    const TileCounts tile_counts{by_tile ? A.tile_counts.p : nullptr, A.pair_cap, cut,
+                                 cut && train ? A.whole.p : nullptr, A.ctrl.p};
+    if (by_tile) zero_words = static_cast<unsigned>(tile_count_words(P.tiles));
     if (ev) AB_CUDA(cudaEventRecord(ev[0], st));
-    const Slot::FrameBegin begin{A.ctrl.p, first.counts, zero_words, A.ranges.p, static_cast<unsigned>(P.tiles)};
+    // The tile sort writes every range itself.
+    const Slot::FrameBegin begin{A.ctrl.p, by_tile ? A.tile_counts.p : first.counts, zero_words, A.ranges.p,
+                                 by_tile ? 0u : tiles};
     AB_TRY(slot.fill(P, st, &views, &scenes, tables, &begin));
-    launch_preprocess_any(scenes, P, views, A, dbg, first, st);
+    launch_preprocess_any(scenes, P, views, A, dbg, first, tile_counts, st);
     if (ev) AB_CUDA(cudaEventRecord(ev[1], st));
     int fin = 0;
-    AB_TRY(enqueue_sort(A, static_cast<unsigned>(P.entries), static_cast<unsigned>(P.tiles), tables, train,
-                        P.shape.radix_bits, first.counts != nullptr, P.short_depth, st, &fin));
+    if (by_tile)
+        enqueue_tile_sort(A, entries, static_cast<unsigned>(P.longest()), tiles, tables, train, st);
+    else
+        AB_TRY(enqueue_sort(A, entries, tiles, tables, train, P.shape.radix_bits, first.counts != nullptr,
+                            P.short_depth, st, &fin));
     if (ev) AB_CUDA(cudaEventRecord(ev[2], st));
     if (!stop_after_sort)
         launch_blend(static_cast<unsigned>(P.tiles), A.ranges.p, A.pair_val[fin].p, A.rec.p, A.ctrl.p, views, tables,
@@ -714,7 +788,7 @@ int settle(Arena& A, const Ctrl& h, int* again, bool all_frames) {
     if (flags & kFlagOverflow) {
         const uint64_t need = pairs + pairs / 4 + 1024;
         if (need > kMaxPairs) return fail(ANISO_B200_ERR_ARGUMENT, "more than 2^30 splat-tile pairs");
-        AB_TRY(A.grow_pairs(static_cast<unsigned>(need)));
+        A.grow_pairs(static_cast<unsigned>(need));
         *again = 1;
     }
     return 0;
@@ -1451,7 +1525,7 @@ int aniso_b200_debug_projection(aniso_b200_scene* s, const aniso_b200_camera* ca
     s->chain.extend(s->stream);
     AB_TRY(slot.fill(P, s->stream, &views, &scenes, tables));
     launch_frame_begin(A.ctrl.p, s->stream);
-    launch_preprocess_any(scenes, P, views, A, &dbg, PassCounts{}, s->stream);
+    launch_preprocess_any(scenes, P, views, A, &dbg, PassCounts{}, TileCounts{}, s->stream);
     AB_TRY(slot.mark(s->stream));
     AB_CUDA(cudaGetLastError());
     AB_CUDA(cudaStreamSynchronize(s->stream));
@@ -1484,10 +1558,12 @@ int aniso_b200_debug_sorted(aniso_b200_scene* s, const aniso_b200_camera* camera
     *pairs = Pn;
     if (Pn > capacity) return fail(ANISO_B200_ERR_ARGUMENT, "capacity too small");
     const Arena& A = s->arena;
-    if (tiles && Pn) AB_CUDA(cudaMemcpy(tiles, A.pair_key[fin].p, Pn * sizeof(unsigned), cudaMemcpyDeviceToHost));
+    std::vector<uint2> r(static_cast<size_t>(P.tiles));
+    AB_CUDA(cudaMemcpy(r.data(), A.ranges.p, r.size() * sizeof(uint2), cudaMemcpyDeviceToHost));
+    if (tiles)  // a tile's pairs are its range
+        for (size_t t = 0; t < r.size(); ++t) std::fill(tiles + r[t].x, tiles + r[t].y, static_cast<uint32_t>(t));
     if (values && Pn) AB_CUDA(cudaMemcpy(values, A.pair_val[fin].p, Pn * sizeof(unsigned), cudaMemcpyDeviceToHost));
-    if (ranges)
-        AB_CUDA(cudaMemcpy(ranges, A.ranges.p, static_cast<size_t>(P.tiles) * sizeof(uint2), cudaMemcpyDeviceToHost));
+    if (ranges) std::memcpy(ranges, r.data(), r.size() * sizeof(uint2));
     return ANISO_B200_OK;
 }
 
@@ -1528,7 +1604,7 @@ int aniso_b200_sort_projection(int64_t n, const uint32_t* tiles_touched, const u
     cudaStream_t st = nullptr;
     const BatchTables tables{dtab.p, dtab.p + 1, dtab.p + 2, 1u};
     const unsigned T = static_cast<unsigned>(tiles_x) * static_cast<unsigned>(tiles_y);
-    AB_TRY(A.reserve_ranges(T));
+    AB_TRY(A.prepare(0, T, 0, false));  // the LSD chain, whatever n
     launch_frame_begin(A.ctrl.p, nullptr, 0u, A.ranges.p, T, st);
     launch_projection_keys(n, dtt.p, ddepth.p, drect.p, A.depth_key.p, A.rect16.p, st,
                            short_depth ? kDepthKeyBase : 0u);
@@ -1646,7 +1722,7 @@ int aniso_b200_batch_render(aniso_b200_batch* b, const aniso_b200_camera* camera
         // pinned blob at every replay, and each replay refreshes that blob first.
         // Every allocation the sequence needs happens first: none may happen while capturing.
         AB_TRY(b->graph_slot.stage(P));
-        AB_TRY(b->arena.reserve_ranges(static_cast<size_t>(P.tiles)));
+        AB_TRY(b->arena.prepare(P.entries, P.tiles, P.longest(), false));
         cudaGraph_t g = nullptr;
         AB_CUDA(cudaStreamBeginCapture(b->capture_stream, cudaStreamCaptureModeThreadLocal));
         const int rc = enqueue_plan(b->arena, b->graph_slot, P, b->capture_stream, nullptr, nullptr, false, false,
@@ -1782,7 +1858,7 @@ int record_graph(aniso_b200_trainer* t, cudaGraphExec_t* exec, F&& enqueue) {
 // the launch geometry or the work buffers changed, else replayed after restaging the graph's slot.
 int train_forward_graph(aniso_b200_trainer* t, const Plan<RawParams>& P, cudaStream_t st, int* fin) {
     Arena& A = t->arena;
-    AB_TRY(A.reserve_ranges(static_cast<size_t>(P.tiles)));
+    AB_TRY(A.prepare(P.entries, P.tiles, P.longest(), true));
     AB_TRY(t->graph_slot_f.stage(P));
     if (!t->fwd_graph || t->fwd_gen != A.gen || !P.same_geometry(t->fwd_plan)) {
         if (t->fwd_graph) {
@@ -1893,6 +1969,11 @@ int train_backward(aniso_b200_trainer* t, const float* const* grad_images, const
         const unsigned s = P.views[k].scene;
         fresh[k] = grads[s].fresh != 0 && k == P.scenes[s].view_begin;
     }
+    // Where the forward's sort left the entries' gradient slots (BackwardIn).
+    const bool by_tile = A.tile_sorted(P.entries, P.tiles);
+    const unsigned* rank = by_tile ? nullptr : A.rank.p;
+    const unsigned long long* rect = by_tile ? A.rect16.p : A.rect_sorted.p;
+    const unsigned long long* whole = by_tile ? A.whole.p : nullptr;
     const auto enqueue = [&](Slot& slot, cudaStream_t cs) -> int {
         const ViewInfo* views = nullptr;
         const BatchScene<RawParams>* scenes = nullptr;
@@ -1903,9 +1984,9 @@ int train_backward(aniso_b200_trainer* t, const float* const* grad_images, const
         in.rec = A.rec.p;
         in.ctrl = A.ctrl.p;
         in.views = views;
-        in.rank = A.rank.p;
+        in.rank = rank;
         in.offs = A.offs.p;
-        in.rect_sorted = A.rect_sorted.p;
+        in.rect = rect;
         AB_CUDA(cudaMemsetAsync(t->vis_counts.p, 0, P.views.size() * sizeof(unsigned), cs));
         launch_blend_backward(in, static_cast<unsigned>(P.tiles), P.shape.tile_w, P.shape.tile_h, t->grad_pair.p, cs);
         for (size_t k = 0; k < P.views.size(); ++k) {
@@ -1913,7 +1994,7 @@ int train_backward(aniso_b200_trainer* t, const float* const* grad_images, const
             const GaussBackwardArgs ga{scenes, s, views, static_cast<unsigned>(k), slot.grads_dev(P),
                                        P.scenes[s].src.n, P.views[k].entry_base, P.views[k].cam.shDegree,
                                        fresh[k] != 0};
-            launch_gauss_backward(ga, A.ctrl.p, A.depth_key.p, A.rank.p, A.offs.p, A.rect_sorted.p, t->grad_pair.p,
+            launch_gauss_backward(ga, A.ctrl.p, A.depth_key.p, rank, A.offs.p, rect, whole, t->grad_pair.p,
                                   t->vis_list.p, t->vis_counts.p + k, cs);
         }
         AB_CUDA(cudaGetLastError());

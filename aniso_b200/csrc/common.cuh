@@ -131,6 +131,42 @@ struct Ctrl {
     unsigned int sort_barrier;          // arrivals at the persistent sort's grid barriers, or CTAs done
                                         // with the tile-bin scan (cleared per frame)
     unsigned long long max_pair_total;  // largest pair_total of earlier frames since then
+    // The tile sort's (sort_tiles.cu), cleared per frame: tiles of the rectangles counted by a whole warp,
+    // entries of the chunk list, gradient slots handed out.
+    unsigned long long large_total;
+    unsigned int chunk_count;
+    unsigned int slot_count;
+};
+
+// Clears the per-frame fields (one thread, at the start of a frame).
+__device__ __forceinline__ void begin_frame(Ctrl* ctrl) {
+    ctrl->sticky_flags |= ctrl->flags;
+    if (ctrl->pair_total > ctrl->max_pair_total) ctrl->max_pair_total = ctrl->pair_total;
+    ctrl->pair_total = 0;
+    ctrl->vis_count = 0;
+    ctrl->flags = 0;
+    ctrl->sort_barrier = 0;
+    ctrl->large_total = 0;
+    ctrl->chunk_count = 0;
+    ctrl->slot_count = 0;
+}
+
+// ---- the tile sort ------------------------------------------------------------------------------
+constexpr unsigned kTileStride = 8;     // words between two counters: one 32-byte sector each
+constexpr unsigned kTileChunk = 2048;   // pairs one CTA sorts in shared memory
+constexpr unsigned kTileGroup = 512;    // chunks of a list that are merged in one step
+constexpr unsigned kWarpArea = 32;      // a rectangle of more tiles is counted by its whole warp
+
+// The tile counts of a frame, accumulated by the preprocess (counts NULL: not wanted). With `cut`, an
+// entry's rectangle is first cut to the tiles that its pixel bounds reach: the tiles that go hold no
+// pixel that could take the splat (28% of all pairs at the 740k / 1280x720 view), so no image and no
+// gradient changes; `full` (training) then keeps the whole rectangles.
+struct TileCounts {
+    unsigned* counts;    // kTileStride words per global tile, zero beforehand
+    unsigned capacity;   // of pairs
+    bool cut;
+    unsigned long long* full;
+    Ctrl* ctrl;
 };
 
 // Depth key of a culled Gaussian. A visible entry's key is its depth's float bits less

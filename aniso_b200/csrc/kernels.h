@@ -39,17 +39,18 @@ void launch_frame_start(const unsigned* src_mapped, unsigned* dst, unsigned word
 // Projection of every (view, Gaussian) entry of a batch; `blocks` = sum over scenes of
 // ceil(n / preprocess_gaussians_per_block()) (scene s starts at block scenes[s].block_base). counts.counts set: each visible
 // entry's depth key is also added to the digit counts of the first depth pass, whose items are the
-// `entries` depth keys in entry order.
+// `entries` depth keys in entry order. tile_counts.counts set: each visible entry's tiles are counted
+// there (launch_tile_sort).
 unsigned preprocess_gaussians_per_block();
 void launch_preprocess(const BatchScene<SceneView>* scenes, unsigned n_scenes, unsigned blocks, const ViewInfo* views,
                        int sh_degree, int tile_w, int tile_h, SplatRecord* rec, unsigned long long* rect16,
                        unsigned* depth_key, const DebugProjection* dbg, const PassCounts& counts, unsigned entries,
-                       cudaStream_t stream);
+                       const TileCounts& tile_counts, cudaStream_t stream);
 // The same projection of the optimizer's raw tensors (activated in the kernel).
 void launch_preprocess_raw(const BatchScene<RawParams>* scenes, unsigned n_scenes, unsigned blocks,
                            const ViewInfo* views, int sh_degree, int tile_w, int tile_h, SplatRecord* rec,
                            unsigned long long* rect16, unsigned* depth_key, const PassCounts& counts,
-                           unsigned entries, cudaStream_t stream);
+                           unsigned entries, const TileCounts& tile_counts, cudaStream_t stream);
 
 // Where a sort pass finds its item count: a host value, the visible count the first depth pass
 // publishes, or the frame's pair total.
@@ -159,6 +160,35 @@ unsigned persistent_sort_ctas();
 size_t persistent_sort_count_words(unsigned ctas);  // words of one count matrix
 cudaError_t launch_sort_frame(const SortFrameArgs& args, unsigned ctas, cudaStream_t stream);
 
+// ---- the tile sort: the same order made per tile (sort_tiles.cu), from the preprocess's tile counts.
+// Writes the sorted entries (vals) and every tile's range; sets kFlagOverflow (and sorts nothing) if
+// the pairs of the preprocess's whole rectangles (Ctrl::pair_total) exceed capacity. offs not NULL: also each
+// visible entry's first gradient slot (a slot per pair, in any order of the entries).
+struct TileSortArgs {
+    const unsigned* depth_key;         // [entries]
+    const unsigned long long* rect16;  // [entries]
+    unsigned entries;
+    unsigned longest;                  // no tile's list is longer (the largest scene's Gaussians)
+    BatchTables tables;
+    unsigned tiles;
+    const unsigned* counts;            // [tile_count_words(tiles)] from the preprocess
+    unsigned* cursor;                  // [tile_count_words(tiles)]
+    unsigned* sums;                    // [tile_sum_words(tiles)]
+    uint2* ranges;                     // [tiles]
+    uint2* chunks;                     // [chunk_cap]: tile_chunk_entries(capacity)
+    unsigned chunk_cap;
+    unsigned long long* pairs;         // [capacity]
+    unsigned long long* merged;        // [capacity] if longest > tile_group_pairs(), else NULL
+    unsigned* vals;                    // [capacity]
+    unsigned* offs;                    // [entries] or NULL
+    unsigned capacity;
+    Ctrl* ctrl;
+};
+size_t tile_count_words(uint64_t tiles);
+size_t tile_sum_words(uint64_t tiles);
+size_t tile_chunk_entries(uint64_t capacity);
+void launch_tile_sort(const TileSortArgs& args, cudaStream_t stream);
+
 // Blends every tile of a batch (blockIdx = global tile); outputs go to each view's ViewInfo.
 // train: also the float colour, final transmittance and last contributor per pixel.
 bool blend_shape_supported(int tile_w, int tile_h);
@@ -174,9 +204,11 @@ struct BackwardIn {
     const Ctrl* ctrl;
     const ViewInfo* views;               // t_final, n_contrib, grad_img per view
     BatchTables tables;
-    const unsigned* rank;                // depth-sorted position of each visible entry
-    const unsigned* offs;                // pair offset of each depth-sorted entry
-    const unsigned long long* rect_sorted;
+    // An entry's gradient slots start at offs[j], its rectangle is rect[j]: j = rank[entry] (the LSD
+    // chain's depth-sorted position), or the entry itself where rank is NULL (the tile sort).
+    const unsigned* rank;
+    const unsigned* offs;
+    const unsigned long long* rect;
 };
 // Gradients of the raw parameters of one scene (device, the layout of RawParams). Added to.
 struct RawGrads {
@@ -208,10 +240,11 @@ struct GaussBackwardArgs {
     int sh_degree;
     bool fresh;
 };
-// The view's visible Gaussians add their gradients to the scene's buffers. list (the scene's n
+// The view's visible Gaussians add their gradients to the scene's buffers. rank, offs, rect as in
+// BackwardIn; whole: the rectangles before they were cut (TileCounts), NULL where they are not. list (the scene's n
 // words) and *list_count (zero on entry) are work space for the compacted visible list.
 void launch_gauss_backward(const GaussBackwardArgs& args, const Ctrl* ctrl, const unsigned* depth_key,
-                           const unsigned* rank, const unsigned* offs, const unsigned long long* rect_sorted,
-                           const float* grad_pair, unsigned* list, unsigned* list_count, cudaStream_t stream);
+                           const unsigned* rank, const unsigned* offs, const unsigned long long* rect,
+                           const unsigned long long* whole, const float* grad_pair, unsigned* list, unsigned* list_count, cudaStream_t stream);
 
 }  // namespace ab2

@@ -254,18 +254,20 @@ constexpr int kPreGaussians = kPreThreads * kPreGroups;  // Gaussians per CTA
 // The projection of one entry that passed the early test, by any lane of the warp (the Gaussian's
 // activated position / opacity and covariance come from its owner lane through shared memory):
 // the exact test, then colour, blend record, rectangle and depth key, all indexed by entry.
+// Returns the rectangle, and whether the entry is visible.
 template <int D, bool kDebug, class Src>
-__device__ __forceinline__ void project_entry(const Src& src, int64_t i, const float4 pg, const Cov3& cov,
+__device__ __forceinline__ bool project_entry(const Src& src, int64_t i, const float4 pg, const Cov3& cov,
                                               const CamParams& cam, unsigned e, int tile_w,
                                               int tile_h, SplatRecord* __restrict__ rec,
                                               unsigned long long* __restrict__ rect16, unsigned* __restrict__ depth_key,
                                               const DebugProjection& dbg, const PassCounts& counts,
-                                              unsigned count_blocks) {
+                                              unsigned count_blocks, const TileCounts& tile_counts,
+                                              unsigned long long& rect, unsigned& whole) {
     Projected p;
     if (!project(pg, cov, cam, tile_w, tile_h, p)) {
         depth_key[e] = kCulledKey;
         if (kDebug) dbg.tiles_touched[e] = 0;
-        return;
+        return false;
     }
     // log2(opacity) for the record. alpha = min(0.99, opacity * exp(power)) >= 1/255 needs
     // power >= -ln(255 opacity) = -ln2 (log2(opacity) + log2(255)): a margin of 1% + 0.02 on that
@@ -290,8 +292,21 @@ __device__ __forceinline__ void project_entry(const Src& src, int64_t i, const f
     r.r1 = make_float4(kHalfLog2e * p.conicC, log2_opacity, rgb.x, rgb.y);
     r.r2 = make_float4(rgb.z, __uint_as_float(bx), __uint_as_float(by), 0.f);
     rec[e] = r;
-    rect16[e] = static_cast<unsigned long long>(p.x0) | (static_cast<unsigned long long>(p.y0) << 16) |
-                (static_cast<unsigned long long>(p.x1) << 32) | (static_cast<unsigned long long>(p.y1) << 48);
+    whole = static_cast<unsigned>((p.x1 - p.x0 + 1) * (p.y1 - p.y0 + 1));
+    const auto pack = [](int x0, int y0, int x1, int y1) {
+        return static_cast<unsigned long long>(x0) | (static_cast<unsigned long long>(y0) << 16) |
+               (static_cast<unsigned long long>(x1) << 32) | (static_cast<unsigned long long>(y1) << 48);
+    };
+    rect = pack(p.x0, p.y0, p.x1, p.y1);
+    if (tile_counts.cut) {  // to the tiles that the pixel bounds reach (none: 1 .. 0, area 0)
+        if (tile_counts.full) tile_counts.full[e] = rect;
+        const int sw = 31 - __clz(tile_w), sh = 31 - __clz(tile_h);  // tile sizes are powers of two
+        const int xlo = unpack_lo(bx), xhi = unpack_hi(bx), ylo = unpack_lo(by), yhi = unpack_hi(by);
+        rect = xlo > xhi || ylo > yhi ? pack(1, 1, 0, 0)
+                                      : pack(max(p.x0, xlo >> sw), max(p.y0, ylo >> sh), min(p.x1, xhi >> sw),
+                                             min(p.y1, yhi >> sh));
+    }
+    rect16[e] = rect;
     // The depth key (the depth's bits less kDepthKeyBase: visible depths are >= 0.2, so the sign
     // bit of kCulledKey never collides). The first depth pass compacts the visible entries.
     const unsigned key = __float_as_uint(p.depth) - kDepthKeyBase;
@@ -306,6 +321,44 @@ __device__ __forceinline__ void project_entry(const Src& src, int64_t i, const f
         dbg.rgb[3 * e + 2] = rgb.z;
         dbg.rect[e] = make_uint4(p.x0, p.y0, p.x1, p.y1);
         dbg.tiles_touched[e] = static_cast<unsigned>((p.x1 - p.x0 + 1) * (p.y1 - p.y0 + 1));
+    }
+    return true;
+}
+
+// Adds one to the count of every tile of the lanes' rectangles (area 0: none), whose corner is global
+// tile org, width w, in a view of tx tiles per row: a small rectangle by its own lane, one of more than
+// kWarpArea tiles by the whole warp, and those only while they can fit the pair capacity (a frame
+// whose large rectangles alone exceed it is not sorted, so their tiles need no counting).
+__device__ __forceinline__ void count_tiles(const TileCounts& tc, unsigned area, unsigned org, unsigned w, unsigned tx,
+                                            int lane) {
+    const bool large = area > kWarpArea;
+    if (!large) {
+        unsigned col = 0, tile = org;
+        for (unsigned k = 0; k < area; ++k) {
+            atomicAdd(&tc.counts[static_cast<size_t>(tile) * kTileStride], 1u);
+            ++tile;
+            if (++col == w) {
+                col = 0;
+                tile += tx - w;
+            }
+        }
+    }
+    unsigned todo = __ballot_sync(0xFFFFFFFFu, large);
+    if (!todo) return;
+    unsigned long long sum = large ? area : 0u;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    int fits = 0;
+    if (lane == 0) fits = atomicAdd(&tc.ctrl->large_total, sum) + sum <= tc.capacity;
+    if (!__shfl_sync(0xFFFFFFFFu, fits, 0)) return;
+    for (; todo; todo &= todo - 1) {
+        const int src = __ffs(todo) - 1;
+        const unsigned n = __shfl_sync(0xFFFFFFFFu, area, src), o = __shfl_sync(0xFFFFFFFFu, org, src),
+                       ow = __shfl_sync(0xFFFFFFFFu, w, src), ot = __shfl_sync(0xFFFFFFFFu, tx, src);
+        for (unsigned k = lane; k < n; k += 32) {
+            const unsigned row = k / ow;
+            atomicAdd(&tc.counts[static_cast<size_t>(o + row * ot + (k - row * ow)) * kTileStride], 1u);
+        }
     }
 }
 
@@ -325,21 +378,25 @@ __global__ void __launch_bounds__(kPreThreads, 4) preprocess_kernel(const BatchS
                                                                     int tile_w, int tile_h, SplatRecord* __restrict__ rec,
                                                                     unsigned long long* __restrict__ rect16,
                                                                     unsigned* __restrict__ depth_key, DebugProjection dbg,
-                                                                    PassCounts counts, unsigned entries) {
+                                                                    PassCounts counts, unsigned entries,
+                                                                    TileCounts tile_counts) {
     chain_entry();
     __shared__ CamParams s_cam[kMaxStagedViews];
-    __shared__ unsigned s_ebase[kMaxStagedViews];
+    __shared__ unsigned s_ebase[kMaxStagedViews], s_tbase[kMaxStagedViews];
     __shared__ unsigned s_queue[kPreWarps][64];
     __shared__ float4 s_pos[kPreWarps][32 * kPreGroups];     // activated position + opacity
     __shared__ float4 s_cova[kPreWarps][32 * kPreGroups];    // s00, s01, s02, s11
     __shared__ float4 s_covb[kPreWarps][32 * kPreGroups];    // s12, s22, trace, splat scale
-    __shared__ unsigned s_scene;
+    __shared__ unsigned s_scene, s_visible;
+    __shared__ unsigned long long s_pairs;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
         unsigned sidx = 0;
         for (unsigned k = 1; k < n_scenes; ++k)
             if (scenes[k].block_base <= blockIdx.x) sidx = k;
         s_scene = sidx;
+        s_visible = 0;
+        s_pairs = 0;
     }
     __syncthreads();
     const BatchScene<Src> sc = scenes[s_scene];
@@ -348,7 +405,10 @@ __global__ void __launch_bounds__(kPreThreads, 4) preprocess_kernel(const BatchS
     for (unsigned k = tid; k < staged * (sizeof(CamParams) / 4); k += kPreThreads)
         reinterpret_cast<unsigned*>(s_cam)[k] =
             reinterpret_cast<const unsigned*>(&views[sc.view_begin + k / (sizeof(CamParams) / 4)].cam)[k % (sizeof(CamParams) / 4)];
-    for (unsigned k = tid; k < staged; k += kPreThreads) s_ebase[k] = views[sc.view_begin + k].entry_base;
+    for (unsigned k = tid; k < staged; k += kPreThreads) {
+        s_ebase[k] = views[sc.view_begin + k].entry_base;
+        s_tbase[k] = views[sc.view_begin + k].tile_base;
+    }
     __syncthreads();
     const unsigned count_blocks = (entries + kSortBlockItems - 1) / kSortBlockItems;
     const int64_t warp_base =
@@ -356,6 +416,8 @@ __global__ void __launch_bounds__(kPreThreads, 4) preprocess_kernel(const BatchS
     unsigned* queue = s_queue[warp];
     const unsigned lt = lanemask_lt();
     unsigned queued = 0;  // items in the warp's queue (warp-uniform)
+    unsigned warp_visible = 0;
+    unsigned long long warp_pairs = 0;
 
     for (int g = 0; g < kPreGroups; ++g) {
         const int64_t i = warp_base + g * 32 + lane;
@@ -409,6 +471,7 @@ __global__ void __launch_bounds__(kPreThreads, 4) preprocess_kernel(const BatchS
             const bool last = g == kPreGroups - 1 && vk == nv;
             while (queued >= 32 || (last && queued > 0)) {
                 const unsigned take = min(queued, 32u);
+                unsigned area = 0, org = 0, width = 1, tx = 0, whole = 0;
                 if (static_cast<unsigned>(lane) < take) {
                     const unsigned item = queue[queued - take + lane];
                     const unsigned ivk = item >> 8;
@@ -424,13 +487,38 @@ __global__ void __launch_bounds__(kPreThreads, 4) preprocess_kernel(const BatchS
                         sc.src.load(gi, pg2, sg, q);
                         covariance(sg, q, cam.splatScale, icov);
                     }
-                    project_entry<D, kDebug>(sc.src, gi, ip, icov, cam, e, tile_w, tile_h, rec, rect16, depth_key, dbg,
-                                             counts, count_blocks);
+                    unsigned long long rect;
+                    if (project_entry<D, kDebug>(sc.src, gi, ip, icov, cam, e, tile_w, tile_h, rec, rect16, depth_key,
+                                                 dbg, counts, count_blocks, tile_counts, rect, whole) &&
+                        tile_counts.counts) {
+                        const unsigned x0 = rect & 0xFFFFu, y0 = (rect >> 16) & 0xFFFFu, x1 = (rect >> 32) & 0xFFFFu;
+                        width = x1 - x0 + 1;  // 0 where nothing is left
+                        tx = static_cast<unsigned>(cam.tilesX);
+                        area = width * (static_cast<unsigned>(rect >> 48) - y0 + 1);
+                        org = (ivk < kMaxStagedViews ? s_tbase[ivk] : views[sc.view_begin + ivk].tile_base) + y0 * tx + x0;
+                    }
+                }
+                if (tile_counts.counts) {
+                    __syncwarp();
+                    warp_visible += __popc(__ballot_sync(0xFFFFFFFFu, whole != 0));
+                    warp_pairs += __reduce_add_sync(0xFFFFFFFFu, whole);
+                    count_tiles(tile_counts, area, org, width, tx, lane);
                 }
                 queued -= take;
                 __syncwarp();
             }
         }
+    }
+    if (!tile_counts.counts) return;
+    // The frame's visible entries and pairs (of whole rectangles): one add per CTA.
+    if (lane == 0) {
+        atomicAdd(&s_visible, warp_visible);
+        atomicAdd(&s_pairs, warp_pairs);
+    }
+    __syncthreads();
+    if (tid == 0 && s_visible) {
+        atomicAdd(&tile_counts.ctrl->vis_count, s_visible);
+        atomicAdd(&tile_counts.ctrl->pair_total, s_pairs);
     }
 }
 
@@ -444,18 +532,19 @@ template <bool kDebug, class Src>
 void launch_preprocess_t(const BatchScene<Src>* scenes, unsigned n_scenes, unsigned blocks, const ViewInfo* views,
                          int sh_degree, int tile_w, int tile_h, SplatRecord* rec,
                          unsigned long long* rect16, unsigned* depth_key, const DebugProjection& dbg,
-                         const PassCounts& counts, unsigned entries, cudaStream_t stream) {
+                         const PassCounts& counts, unsigned entries, const TileCounts& tile_counts,
+                         cudaStream_t stream) {
     if (blocks == 0) return;
     const dim3 grid(blocks), block(kPreThreads);
     switch (sh_degree) {
         case 0: launch_chained(preprocess_kernel<0, kDebug, Src>, grid, block, stream, scenes, n_scenes, views, tile_w,
-                               tile_h, rec, rect16, depth_key, dbg, counts, entries); break;
+                               tile_h, rec, rect16, depth_key, dbg, counts, entries, tile_counts); break;
         case 1: launch_chained(preprocess_kernel<1, kDebug, Src>, grid, block, stream, scenes, n_scenes, views, tile_w,
-                               tile_h, rec, rect16, depth_key, dbg, counts, entries); break;
+                               tile_h, rec, rect16, depth_key, dbg, counts, entries, tile_counts); break;
         case 2: launch_chained(preprocess_kernel<2, kDebug, Src>, grid, block, stream, scenes, n_scenes, views, tile_w,
-                               tile_h, rec, rect16, depth_key, dbg, counts, entries); break;
+                               tile_h, rec, rect16, depth_key, dbg, counts, entries, tile_counts); break;
         default: launch_chained(preprocess_kernel<3, kDebug, Src>, grid, block, stream, scenes, n_scenes, views, tile_w,
-                                tile_h, rec, rect16, depth_key, dbg, counts, entries); break;
+                                tile_h, rec, rect16, depth_key, dbg, counts, entries, tile_counts); break;
     }
 }
 
@@ -464,21 +553,21 @@ void launch_preprocess_t(const BatchScene<Src>* scenes, unsigned n_scenes, unsig
 void launch_preprocess(const BatchScene<SceneView>* scenes, unsigned n_scenes, unsigned blocks, const ViewInfo* views,
                        int sh_degree, int tile_w, int tile_h, SplatRecord* rec, unsigned long long* rect16,
                        unsigned* depth_key, const DebugProjection* dbg, const PassCounts& counts, unsigned entries,
-                       cudaStream_t stream) {
+                       const TileCounts& tile_counts, cudaStream_t stream) {
     if (dbg)
         launch_preprocess_t<true>(scenes, n_scenes, blocks, views, sh_degree, tile_w, tile_h, rec, rect16,
-                                  depth_key, *dbg, counts, entries, stream);
+                                  depth_key, *dbg, counts, entries, tile_counts, stream);
     else
         launch_preprocess_t<false>(scenes, n_scenes, blocks, views, sh_degree, tile_w, tile_h, rec, rect16,
-                                   depth_key, DebugProjection{}, counts, entries, stream);
+                                   depth_key, DebugProjection{}, counts, entries, tile_counts, stream);
 }
 
 void launch_preprocess_raw(const BatchScene<RawParams>* scenes, unsigned n_scenes, unsigned blocks,
                            const ViewInfo* views, int sh_degree, int tile_w, int tile_h, SplatRecord* rec,
                            unsigned long long* rect16, unsigned* depth_key, const PassCounts& counts,
-                           unsigned entries, cudaStream_t stream) {
+                           unsigned entries, const TileCounts& tile_counts, cudaStream_t stream) {
     launch_preprocess_t<false>(scenes, n_scenes, blocks, views, sh_degree, tile_w, tile_h, rec, rect16,
-                               depth_key, DebugProjection{}, counts, entries, stream);
+                               depth_key, DebugProjection{}, counts, entries, tile_counts, stream);
 }
 
 }  // namespace ab2

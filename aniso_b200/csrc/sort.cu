@@ -60,16 +60,9 @@ static_assert(kExpandChunk == kSortBlockItems, "an expansion CTA writes exactly 
 __global__ void frame_begin_kernel(Ctrl* ctrl, unsigned* __restrict__ zero, unsigned zero_words,
                                    uint2* __restrict__ range, unsigned ranges) {
     chain_entry();
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ctrl->sticky_flags |= ctrl->flags;
-        if (ctrl->pair_total > ctrl->max_pair_total) ctrl->max_pair_total = ctrl->pair_total;
-        ctrl->pair_total = 0;
-        ctrl->vis_count = 0;
-        ctrl->flags = 0;
-        ctrl->sort_barrier = 0;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) begin_frame(ctrl);
     const unsigned stride = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
-    for (unsigned i = first; i < zero_words; i += stride) zero[i] = 0;  // at most 512 x 592 words
+    for (unsigned long long i = first; i < zero_words; i += stride) zero[i] = 0;
     // 64-bit index: a tile count within one stride of 2^32 must not wrap the loop.
     for (unsigned long long i = first; i < ranges; i += stride) range[i] = make_uint2(0u, 0u);
 }
@@ -93,15 +86,8 @@ __global__ void frame_start_kernel(const unsigned* __restrict__ src, unsigned* _
     chain_entry();
     const unsigned stride = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
     for (unsigned i = first; i < words; i += stride) dst[i] = __ldcv(src + i);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ctrl->sticky_flags |= ctrl->flags;
-        if (ctrl->pair_total > ctrl->max_pair_total) ctrl->max_pair_total = ctrl->pair_total;
-        ctrl->pair_total = 0;
-        ctrl->vis_count = 0;
-        ctrl->flags = 0;
-        ctrl->sort_barrier = 0;
-    }
-    for (unsigned i = first; i < zero_words; i += stride) zero[i] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) begin_frame(ctrl);
+    for (unsigned long long i = first; i < zero_words; i += stride) zero[i] = 0;
     for (unsigned long long i = first; i < ranges; i += stride) range[i] = make_uint2(0u, 0u);
 }
 
@@ -1009,7 +995,7 @@ void launch_upload(const unsigned* src_mapped, unsigned* dst, unsigned words, cu
 void launch_frame_start(const unsigned* src_mapped, unsigned* dst, unsigned words, Ctrl* ctrl, unsigned* zero,
                         unsigned zero_words, uint2* ranges, unsigned tiles, cudaStream_t stream) {
     const unsigned most = std::max(std::max(zero_words, tiles), words);
-    const unsigned blocks = std::max(1u, std::min((most + kThreads * 4 - 1) / (kThreads * 4), 148u));
+    const unsigned blocks = std::max(1u, std::min(most / (kThreads * 4) + 1, 148u * 4u));
     launch_chained(frame_start_kernel, dim3(blocks), dim3(kThreads), stream, src_mapped, dst, words, ctrl, zero,
                    zero_words, ranges, tiles);
 }
