@@ -36,18 +36,19 @@ void launch_frame_begin(Ctrl* ctrl, unsigned* zero, unsigned zero_words, uint2* 
 void launch_frame_start(const unsigned* src_mapped, unsigned* dst, unsigned words, Ctrl* ctrl, unsigned* zero,
                         unsigned zero_words, uint2* ranges, unsigned tiles, cudaStream_t stream);
 
-// Projection of every (view, Gaussian) entry of a batch; `blocks` = sum over scenes of
-// ceil(n / preprocess_gaussians_per_block()) (scene s starts at block scenes[s].block_base). counts.counts set: each visible
+// Projection of every (view, Gaussian) entry of a batch, `groups` (1 or 2) Gaussians per thread; `blocks` =
+// sum over scenes of ceil(n / preprocess_gaussians_per_block(groups)) (scene s starts at block
+// scenes[s].block_base). counts.counts set: each visible
 // entry's depth key is also added to the digit counts of the first depth pass, whose items are the
 // `entries` depth keys in entry order. tile_counts.counts set: each visible entry's tiles are counted
 // there (launch_tile_sort).
-unsigned preprocess_gaussians_per_block();
-void launch_preprocess(const BatchScene<SceneView>* scenes, unsigned n_scenes, unsigned blocks, const ViewInfo* views,
-                       int sh_degree, int tile_w, int tile_h, SplatRecord* rec, unsigned long long* rect16,
-                       unsigned* depth_key, const DebugProjection* dbg, const PassCounts& counts, unsigned entries,
-                       const TileCounts& tile_counts, cudaStream_t stream);
+unsigned preprocess_gaussians_per_block(int groups);
+void launch_preprocess(const BatchScene<SceneView>* scenes, unsigned n_scenes, unsigned blocks, int groups,
+                       const ViewInfo* views, int sh_degree, int tile_w, int tile_h, SplatRecord* rec,
+                       unsigned long long* rect16, unsigned* depth_key, const DebugProjection* dbg,
+                       const PassCounts& counts, unsigned entries, const TileCounts& tile_counts, cudaStream_t stream);
 // The same projection of the optimizer's raw tensors (activated in the kernel).
-void launch_preprocess_raw(const BatchScene<RawParams>* scenes, unsigned n_scenes, unsigned blocks,
+void launch_preprocess_raw(const BatchScene<RawParams>* scenes, unsigned n_scenes, unsigned blocks, int groups,
                            const ViewInfo* views, int sh_degree, int tile_w, int tile_h, SplatRecord* rec,
                            unsigned long long* rect16, unsigned* depth_key, const PassCounts& counts,
                            unsigned entries, const TileCounts& tile_counts, cudaStream_t stream);

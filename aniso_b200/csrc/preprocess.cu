@@ -246,10 +246,10 @@ __device__ __forceinline__ unsigned axis_bounds(float centre, float cov, float t
 }
 
 constexpr int kMaxStagedViews = 64;  // cameras of a scene's views kept in shared memory
-constexpr int kPreThreads = 256;
+constexpr int kPreThreads = 128;
 constexpr int kPreWarps = kPreThreads / 32;
-constexpr int kPreGroups = 1;  // groups of 32 Gaussians each warp tests (2 and 4 measured slower)
-constexpr int kPreGaussians = kPreThreads * kPreGroups;  // Gaussians per CTA
+constexpr int kPreSlotBits = 10;  // of a queue item: the Gaussian's place in the CTA; the view above it
+static_assert(2 * kPreThreads <= 1 << kPreSlotBits, "a place fits its bits");
 
 // The projection of one entry that passed the early test, by any lane of the warp (the Gaussian's
 // activated position / opacity and covariance come from its owner lane through shared memory):
@@ -362,18 +362,24 @@ __device__ __forceinline__ void count_tiles(const TileCounts& tc, unsigned area,
     }
 }
 
-// Every (view, Gaussian) entry of a scene's views. Each warp owns kPreGroups x 32 Gaussians. For
-// each group it reads the 32 Gaussians once (one per lane) and runs the early screen test of
-// project() for every view of the scene; entries that fail it are written culled at once, the
-// others are queued in shared memory as (Gaussian, view) items. Whenever 32 items are queued the
-// whole warp projects them, one per lane (project_entry), so the expensive part -- the exact
-// test, the SH colour, the record -- runs without idle lanes however the visible entries are
-// spread over the Gaussians and views (a quarter of the entries of a 64-view batch are visible,
-// scattered over every warp). Outputs are indexed by entry, so the queue order does not matter.
-// The kernel is latency-bound, so it is held to 64 registers for four CTAs per SM. Measured: the
-// 64-view batch 10.2 -> 9.5 ms per batch, the 740k view 0.350 -> 0.344 ms per frame.
-template <int D, bool kDebug, class Src>
-__global__ void __launch_bounds__(kPreThreads, 4) preprocess_kernel(const BatchScene<Src>* __restrict__ scenes,
+// Every (view, Gaussian) entry of a scene's views. A CTA reads kPreGroups Gaussians per thread once and
+// runs the early screen test of project() for every view of the scene; entries that fail it are
+// written culled at once, the others are queued per warp in shared memory as (Gaussian, view) items.
+// Whenever a warp has 32 items queued it projects them, one per lane (project_entry); when it has
+// nothing left to test, the CTA's warps put what is left in their queues together and share it out
+// again in full warps. So the expensive part -- the exact test, the SH colour, the record, the tile
+// counts -- runs without idle lanes however the visible entries are spread, also in a single view,
+// where a warp's own 32 Gaussians have 14 visible on average. Outputs are indexed by entry, so the queue
+// order does not matter.
+//
+// Latency-bound (52% issue-active), held to 64 registers for eight CTAs of 128 threads per SM. Measured
+// at 2.2M / 1920x1080 (frame): 447 us with per-warp queues only, 430 us with the last items shared out
+// over 256 threads, 407 us with two Gaussians per thread (more of the warps have items to project),
+// 402 us with 128 threads (shorter waits for the CTA's slowest warp); at 740k / 1280x720: 198, 195, 195,
+// 191 us. Four Gaussians per thread, 64 threads, or 80 registers: slower. Persistent CTAs that take
+// blocks in turn: slower too (446 us; spills).
+template <int D, int kPreGroups, bool kDebug, class Src>
+__global__ void __launch_bounds__(kPreThreads, 8) preprocess_kernel(const BatchScene<Src>* __restrict__ scenes,
                                                                     unsigned n_scenes, const ViewInfo* __restrict__ views,
                                                                     int tile_w, int tile_h, SplatRecord* __restrict__ rec,
                                                                     unsigned long long* __restrict__ rect16,
@@ -381,13 +387,15 @@ __global__ void __launch_bounds__(kPreThreads, 4) preprocess_kernel(const BatchS
                                                                     PassCounts counts, unsigned entries,
                                                                     TileCounts tile_counts) {
     chain_entry();
+    constexpr int kPreGaussians = kPreThreads * kPreGroups;  // of a CTA
     __shared__ CamParams s_cam[kMaxStagedViews];
     __shared__ unsigned s_ebase[kMaxStagedViews], s_tbase[kMaxStagedViews];
     __shared__ unsigned s_queue[kPreWarps][64];
-    __shared__ float4 s_pos[kPreWarps][32 * kPreGroups];     // activated position + opacity
-    __shared__ float4 s_cova[kPreWarps][32 * kPreGroups];    // s00, s01, s02, s11
-    __shared__ float4 s_covb[kPreWarps][32 * kPreGroups];    // s12, s22, trace, splat scale
-    __shared__ unsigned s_scene, s_visible;
+    __shared__ unsigned s_merged[kPreThreads];                // the warps' last items, together
+    __shared__ float4 s_pos[kPreGaussians];     // activated position + opacity
+    __shared__ float4 s_cova[kPreGaussians];    // s00, s01, s02, s11
+    __shared__ float4 s_covb[kPreGaussians];    // s12, s22, trace, splat scale
+    __shared__ unsigned s_scene, s_merged_count, s_visible;
     __shared__ unsigned long long s_pairs;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
@@ -395,6 +403,7 @@ __global__ void __launch_bounds__(kPreThreads, 4) preprocess_kernel(const BatchS
         for (unsigned k = 1; k < n_scenes; ++k)
             if (scenes[k].block_base <= blockIdx.x) sidx = k;
         s_scene = sidx;
+        s_merged_count = 0;
         s_visible = 0;
         s_pairs = 0;
     }
@@ -411,104 +420,124 @@ __global__ void __launch_bounds__(kPreThreads, 4) preprocess_kernel(const BatchS
     }
     __syncthreads();
     const unsigned count_blocks = (entries + kSortBlockItems - 1) / kSortBlockItems;
-    const int64_t warp_base =
-        static_cast<int64_t>(blockIdx.x - sc.block_base) * kPreGaussians + static_cast<int64_t>(warp) * 32 * kPreGroups;
+    const int64_t block_first = static_cast<int64_t>(blockIdx.x - sc.block_base) * kPreGaussians;
     unsigned* queue = s_queue[warp];
     const unsigned lt = lanemask_lt();
     unsigned queued = 0;  // items in the warp's queue (warp-uniform)
     unsigned warp_visible = 0;
     unsigned long long warp_pairs = 0;
 
-    for (int g = 0; g < kPreGroups; ++g) {
-        const int64_t i = warp_base + g * 32 + lane;
-        const bool have = i < sc.src.n;
-        float4 pg = make_float4(0.f, 0.f, 0.f, 0.f);
-        Cov3 cov{};
-        float cov_scale = 0.f;
-        bool prefetched = false;
-        if (have) {
-            float4 sg, q;
-            sc.src.load(i, pg, sg, q);
-            cov_scale = nv > 0 ? s_cam[0].splatScale : 1.0f;
-            covariance(sg, q, cov_scale, cov);
+    // The thread's Gaussians, kPreThreads apart: all loads first.
+    {
+        float4 pg[kPreGroups], sg[kPreGroups], q[kPreGroups];
+#pragma unroll
+        for (int g = 0; g < kPreGroups; ++g) {
+            const int64_t i = block_first + g * kPreThreads + tid;
+            pg[g] = sg[g] = q[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i < sc.src.n) sc.src.load(i, pg[g], sg[g], q[g]);
         }
-        s_pos[warp][g * 32 + lane] = pg;
-        s_cova[warp][g * 32 + lane] = make_float4(cov.s00, cov.s01, cov.s02, cov.s11);
-        s_covb[warp][g * 32 + lane] = make_float4(cov.s12, cov.s22, cov.trace, cov_scale);
-        for (unsigned vk = 0; vk < nv;) {
-            // Test views until the queue holds a warp's worth of items (or the views run out).
-            for (; vk < nv && queued < 32; ++vk) {
-                const CamParams& cam = vk < kMaxStagedViews ? s_cam[vk] : views[sc.view_begin + vk].cam;
-                bool pass = false;
-                if (have) {
-                    if (cam.splatScale != cov_scale) {
-                        float4 pg2, sg, q;
-                        sc.src.load(i, pg2, sg, q);
-                        cov_scale = cam.splatScale;
-                        covariance(sg, q, cov_scale, cov);
-                    }
-                    pass = early_visible(pg, cov, cam);
-                    if (!pass) {
-                        const unsigned e = (vk < kMaxStagedViews ? s_ebase[vk] : views[sc.view_begin + vk].entry_base) +
-                                           static_cast<unsigned>(i);
-                        depth_key[e] = kCulledKey;
-                        if (kDebug) dbg.tiles_touched[e] = 0;
-                    } else if (!prefetched) {
-                        // Its SH words start towards L2 now; the warp projects it later.
-                        const char* shp = reinterpret_cast<const char*>(sc.src.sh + i * sc.src.sh_planes);
-                        for (int off = 0; off < sc.src.sh_planes * 16; off += 128)
-                            asm volatile("prefetch.global.L2 [%0];" ::"l"(shp + off));
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(shp + sc.src.sh_planes * 16 - 1));
-                        prefetched = true;
-                    }
-                }
-                const unsigned m = __ballot_sync(0xFFFFFFFFu, pass);
-                if (pass) queue[queued + __popc(m & lt)] = static_cast<unsigned>(g * 32 + lane) | (vk << 8);
-                queued += __popc(m);
-            }
-            __syncwarp();
-            // A full warp of items (or, after the last group, what is left) is projected.
-            const bool last = g == kPreGroups - 1 && vk == nv;
-            while (queued >= 32 || (last && queued > 0)) {
-                const unsigned take = min(queued, 32u);
-                unsigned area = 0, org = 0, width = 1, tx = 0, whole = 0;
-                if (static_cast<unsigned>(lane) < take) {
-                    const unsigned item = queue[queued - take + lane];
-                    const unsigned ivk = item >> 8;
-                    const int64_t gi = warp_base + (item & 0xFFu);
-                    const CamParams& cam = ivk < kMaxStagedViews ? s_cam[ivk] : views[sc.view_begin + ivk].cam;
-                    const unsigned e = (ivk < kMaxStagedViews ? s_ebase[ivk] : views[sc.view_begin + ivk].entry_base) +
-                                       static_cast<unsigned>(gi);
-                    const float4 ip = s_pos[warp][item & 0xFFu];
-                    const float4 ca = s_cova[warp][item & 0xFFu], cb = s_covb[warp][item & 0xFFu];
-                    Cov3 icov{ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z};
-                    if (cam.splatScale != cb.w) {  // a view with another splat scale than the first
-                        float4 pg2, sg, q;
-                        sc.src.load(gi, pg2, sg, q);
-                        covariance(sg, q, cam.splatScale, icov);
-                    }
-                    unsigned long long rect;
-                    if (project_entry<D, kDebug>(sc.src, gi, ip, icov, cam, e, tile_w, tile_h, rec, rect16, depth_key,
-                                                 dbg, counts, count_blocks, tile_counts, rect, whole) &&
-                        tile_counts.counts) {
-                        const unsigned x0 = rect & 0xFFFFu, y0 = (rect >> 16) & 0xFFFFu, x1 = (rect >> 32) & 0xFFFFu;
-                        width = x1 - x0 + 1;  // 0 where nothing is left
-                        tx = static_cast<unsigned>(cam.tilesX);
-                        area = width * (static_cast<unsigned>(rect >> 48) - y0 + 1);
-                        org = (ivk < kMaxStagedViews ? s_tbase[ivk] : views[sc.view_begin + ivk].tile_base) + y0 * tx + x0;
-                    }
-                }
-                if (tile_counts.counts) {
-                    __syncwarp();
-                    warp_visible += __popc(__ballot_sync(0xFFFFFFFFu, whole != 0));
-                    warp_pairs += __reduce_add_sync(0xFFFFFFFFu, whole);
-                    count_tiles(tile_counts, area, org, width, tx, lane);
-                }
-                queued -= take;
-                __syncwarp();
-            }
+        const float scale = nv > 0 ? s_cam[0].splatScale : 1.0f;
+#pragma unroll
+        for (int g = 0; g < kPreGroups; ++g) {
+            Cov3 cov;
+            covariance(sg[g], q[g], scale, cov);
+            s_pos[g * kPreThreads + tid] = pg[g];
+            s_cova[g * kPreThreads + tid] = make_float4(cov.s00, cov.s01, cov.s02, cov.s11);
+            s_covb[g * kPreThreads + tid] = make_float4(cov.s12, cov.s22, cov.trace, scale);
         }
     }
+    // The covariance of the block's Gaussian `slot` for a view: from shared memory, or made again for a
+    // view with another splat scale than the first.
+    const auto cov_of = [&](unsigned slot, const CamParams& cam) {
+        const float4 ca = s_cova[slot], cb = s_covb[slot];
+        Cov3 cov{ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z};
+        if (cam.splatScale != cb.w) {
+            float4 pg2, sg, q;
+            sc.src.load(block_first + slot, pg2, sg, q);
+            covariance(sg, q, cam.splatScale, cov);
+        }
+        return cov;
+    };
+
+    unsigned vk = 0, group = 0;  // the next (view, group) to test
+    unsigned prefetched = 0;     // bit g: the SH words of the thread's Gaussian g are on their way
+    bool last = false;
+    do {
+        // Test until the queue holds a warp's worth of items (or nothing is left to test).
+        while (vk < nv && queued < 32) {
+            const CamParams& cam = vk < kMaxStagedViews ? s_cam[vk] : views[sc.view_begin + vk].cam;
+            const unsigned slot = group * kPreThreads + tid;
+            const int64_t i = block_first + slot;
+            bool pass = false;
+            if (i < sc.src.n) {
+                pass = early_visible(s_pos[slot], cov_of(slot, cam), cam);
+                if (!pass) {
+                    const unsigned e = (vk < kMaxStagedViews ? s_ebase[vk] : views[sc.view_begin + vk].entry_base) +
+                                       static_cast<unsigned>(i);
+                    depth_key[e] = kCulledKey;
+                    if (kDebug) dbg.tiles_touched[e] = 0;
+                } else if (!((prefetched >> group) & 1u)) {
+                    // Its SH words start towards L2 now; a warp projects it later.
+                    const char* shp = reinterpret_cast<const char*>(sc.src.sh + i * sc.src.sh_planes);
+                    for (int off = 0; off < sc.src.sh_planes * 16; off += 128)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(shp + off));
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(shp + sc.src.sh_planes * 16 - 1));
+                    prefetched |= 1u << group;
+                }
+            }
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, pass);
+            if (pass) queue[queued + __popc(m & lt)] = slot | (vk << kPreSlotBits);
+            queued += __popc(m);
+            if (++group == kPreGroups) {
+                group = 0;
+                ++vk;
+            }
+        }
+        __syncwarp();
+        unsigned take = 32, item = 0;
+        if (queued >= 32) {
+            queued -= 32;
+            item = queue[queued + lane];
+        } else {
+            // Nothing left to test: what is left in the warps' queues is shared out again in full warps.
+            last = true;
+            unsigned at = 0;
+            if (lane == 0) at = atomicAdd(&s_merged_count, queued);
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            if (static_cast<unsigned>(lane) < queued) s_merged[at + lane] = queue[lane];
+            __syncthreads();
+            const unsigned total = s_merged_count, first = warp * 32u;
+            take = total > first ? min(total - first, 32u) : 0u;
+            if (static_cast<unsigned>(lane) < take) item = s_merged[first + lane];
+        }
+        if (take) {
+            unsigned area = 0, org = 0, width = 1, tx = 0, whole = 0;
+            if (static_cast<unsigned>(lane) < take) {
+                const unsigned ivk = item >> kPreSlotBits, slot = item & ((1u << kPreSlotBits) - 1);
+                const int64_t gi = block_first + slot;
+                const CamParams& cam = ivk < kMaxStagedViews ? s_cam[ivk] : views[sc.view_begin + ivk].cam;
+                const unsigned e = (ivk < kMaxStagedViews ? s_ebase[ivk] : views[sc.view_begin + ivk].entry_base) +
+                                   static_cast<unsigned>(gi);
+                unsigned long long rect;
+                if (project_entry<D, kDebug>(sc.src, gi, s_pos[slot], cov_of(slot, cam), cam, e, tile_w, tile_h, rec,
+                                             rect16, depth_key, dbg, counts, count_blocks, tile_counts, rect, whole) &&
+                    tile_counts.counts) {
+                    const unsigned x0 = rect & 0xFFFFu, y0 = (rect >> 16) & 0xFFFFu, x1 = (rect >> 32) & 0xFFFFu;
+                    width = x1 - x0 + 1;  // 0 where nothing is left
+                    tx = static_cast<unsigned>(cam.tilesX);
+                    area = width * (static_cast<unsigned>(rect >> 48) - y0 + 1);
+                    org = (ivk < kMaxStagedViews ? s_tbase[ivk] : views[sc.view_begin + ivk].tile_base) + y0 * tx + x0;
+                }
+            }
+            if (tile_counts.counts) {
+                __syncwarp();
+                warp_visible += __popc(__ballot_sync(0xFFFFFFFFu, whole != 0));
+                warp_pairs += __reduce_add_sync(0xFFFFFFFFu, whole);
+                count_tiles(tile_counts, area, org, width, tx, lane);
+            }
+        }
+        __syncwarp();
+    } while (!last);
     if (!tile_counts.counts) return;
     // The frame's visible entries and pairs (of whole rectangles): one add per CTA.
     if (lane == 0) {
@@ -524,11 +553,11 @@ __global__ void __launch_bounds__(kPreThreads, 4) preprocess_kernel(const BatchS
 
 }  // namespace
 
-unsigned preprocess_gaussians_per_block() { return kPreGaussians; }
+unsigned preprocess_gaussians_per_block(int groups) { return kPreThreads * groups; }
 
 namespace {
 
-template <bool kDebug, class Src>
+template <int G, bool kDebug, class Src>
 void launch_preprocess_t(const BatchScene<Src>* scenes, unsigned n_scenes, unsigned blocks, const ViewInfo* views,
                          int sh_degree, int tile_w, int tile_h, SplatRecord* rec,
                          unsigned long long* rect16, unsigned* depth_key, const DebugProjection& dbg,
@@ -536,38 +565,38 @@ void launch_preprocess_t(const BatchScene<Src>* scenes, unsigned n_scenes, unsig
                          cudaStream_t stream) {
     if (blocks == 0) return;
     const dim3 grid(blocks), block(kPreThreads);
-    switch (sh_degree) {
-        case 0: launch_chained(preprocess_kernel<0, kDebug, Src>, grid, block, stream, scenes, n_scenes, views, tile_w,
-                               tile_h, rec, rect16, depth_key, dbg, counts, entries, tile_counts); break;
-        case 1: launch_chained(preprocess_kernel<1, kDebug, Src>, grid, block, stream, scenes, n_scenes, views, tile_w,
-                               tile_h, rec, rect16, depth_key, dbg, counts, entries, tile_counts); break;
-        case 2: launch_chained(preprocess_kernel<2, kDebug, Src>, grid, block, stream, scenes, n_scenes, views, tile_w,
-                               tile_h, rec, rect16, depth_key, dbg, counts, entries, tile_counts); break;
-        default: launch_chained(preprocess_kernel<3, kDebug, Src>, grid, block, stream, scenes, n_scenes, views, tile_w,
-                                tile_h, rec, rect16, depth_key, dbg, counts, entries, tile_counts); break;
-    }
+    const auto kernel = sh_degree <= 0   ? preprocess_kernel<0, G, kDebug, Src>
+                        : sh_degree == 1 ? preprocess_kernel<1, G, kDebug, Src>
+                        : sh_degree == 2 ? preprocess_kernel<2, G, kDebug, Src>
+                                         : preprocess_kernel<3, G, kDebug, Src>;
+    launch_chained(kernel, grid, block, stream, scenes, n_scenes, views, tile_w, tile_h, rec, rect16, depth_key, dbg,
+                   counts, entries, tile_counts);
 }
 
 }  // namespace
 
-void launch_preprocess(const BatchScene<SceneView>* scenes, unsigned n_scenes, unsigned blocks, const ViewInfo* views,
-                       int sh_degree, int tile_w, int tile_h, SplatRecord* rec, unsigned long long* rect16,
-                       unsigned* depth_key, const DebugProjection* dbg, const PassCounts& counts, unsigned entries,
-                       const TileCounts& tile_counts, cudaStream_t stream) {
-    if (dbg)
-        launch_preprocess_t<true>(scenes, n_scenes, blocks, views, sh_degree, tile_w, tile_h, rec, rect16,
-                                  depth_key, *dbg, counts, entries, tile_counts, stream);
-    else
-        launch_preprocess_t<false>(scenes, n_scenes, blocks, views, sh_degree, tile_w, tile_h, rec, rect16,
-                                   depth_key, DebugProjection{}, counts, entries, tile_counts, stream);
+void launch_preprocess(const BatchScene<SceneView>* scenes, unsigned n_scenes, unsigned blocks, int groups,
+                       const ViewInfo* views, int sh_degree, int tile_w, int tile_h, SplatRecord* rec,
+                       unsigned long long* rect16, unsigned* depth_key, const DebugProjection* dbg,
+                       const PassCounts& counts, unsigned entries, const TileCounts& tile_counts, cudaStream_t stream) {
+    if (dbg) {
+        const auto launch = groups == 2 ? launch_preprocess_t<2, true, SceneView> : launch_preprocess_t<1, true, SceneView>;
+        launch(scenes, n_scenes, blocks, views, sh_degree, tile_w, tile_h, rec, rect16, depth_key, *dbg, counts, entries,
+               tile_counts, stream);
+    } else {
+        const auto launch = groups == 2 ? launch_preprocess_t<2, false, SceneView> : launch_preprocess_t<1, false, SceneView>;
+        launch(scenes, n_scenes, blocks, views, sh_degree, tile_w, tile_h, rec, rect16, depth_key, DebugProjection{},
+               counts, entries, tile_counts, stream);
+    }
 }
 
-void launch_preprocess_raw(const BatchScene<RawParams>* scenes, unsigned n_scenes, unsigned blocks,
+void launch_preprocess_raw(const BatchScene<RawParams>* scenes, unsigned n_scenes, unsigned blocks, int groups,
                            const ViewInfo* views, int sh_degree, int tile_w, int tile_h, SplatRecord* rec,
                            unsigned long long* rect16, unsigned* depth_key, const PassCounts& counts,
                            unsigned entries, const TileCounts& tile_counts, cudaStream_t stream) {
-    launch_preprocess_t<false>(scenes, n_scenes, blocks, views, sh_degree, tile_w, tile_h, rec, rect16,
-                               depth_key, DebugProjection{}, counts, entries, tile_counts, stream);
+    const auto launch = groups == 2 ? launch_preprocess_t<2, false, RawParams> : launch_preprocess_t<1, false, RawParams>;
+    launch(scenes, n_scenes, blocks, views, sh_degree, tile_w, tile_h, rec, rect16, depth_key, DebugProjection{}, counts,
+           entries, tile_counts, stream);
 }
 
 }  // namespace ab2
