@@ -17,8 +17,9 @@
 // 1280x720), 536 -> 483 us (2.2M, 1920x1080), the 64-view 1M batch 7.35 -> 7.04 ms; with the rectangles
 // cut 47, 197, 447 us and 6.42 ms.
 //
-// No CTA waits on another. What bounds the parts: the scatter the adds on the tiles' counters (about
-// 50 a nanosecond over the chip), the sort and the scan latency. The counters lie kTileStride words
+// No CTA waits on another. What bounds the parts: the scatter its scattered accesses (an add and an
+// 8-byte store per pair, each a sector of its own: 46 pairs a nanosecond over the chip), the sort and
+// the scan latency. The counters lie kTileStride words
 // apart: neighbouring tiles are hit together (the 100k view takes 72, 59, 55, 53 us at 1, 2, 4, 8 words;
 // several counters per tile, to spread the adds further, cost the scan more than they gave).
 #include <algorithm>
@@ -41,49 +42,20 @@ constexpr unsigned kScanTiles = kScanThreads * kScanPer;  // tiles per scan CTA
 // leaves each CTA's total first.
 constexpr unsigned kScanDirect = 1u << 16;
 
-// Exclusive prefix of the threads' values over the CTA and their total, in 64 bits (a frame that
-// overflows may count more than 32 hold).
-__device__ __forceinline__ unsigned long long scan_u64(unsigned long long v, unsigned long long* s_tmp,
-                                                       unsigned long long& total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned long long incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) s_tmp[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        unsigned long long x = s_tmp[lane];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-            if (lane >= o) x += y;
-        }
-        s_tmp[lane] = x;
-    }
-    __syncthreads();
-    total = s_tmp[31];
-    const unsigned long long before = warp ? s_tmp[warp - 1] : 0ull;
-    __syncthreads();
-    return before + incl - v;
-}
-
 // sums[b] = pairs of tiles [b kScanTiles, (b + 1) kScanTiles).
 __global__ void __launch_bounds__(kScanThreads) tile_sums_kernel(const unsigned* __restrict__ counts, unsigned tiles,
                                                                  unsigned* __restrict__ sums) {
     chain_entry();
-    __shared__ unsigned long long s_tmp[kScanThreads / 32];
-    unsigned long long v = 0;
+    __shared__ unsigned s_tmp[kScanThreads / 32];
+    unsigned v = 0;
 #pragma unroll
     for (int k = 0; k < kScanPer; ++k) {
         const unsigned long long t = static_cast<unsigned long long>(blockIdx.x) * kScanTiles + k * kScanThreads + threadIdx.x;
         if (t < tiles) v += counts[t * static_cast<size_t>(kTileStride)];
     }
-    unsigned long long total;
-    scan_u64(v, s_tmp, total);
-    if (threadIdx.x == 0) sums[blockIdx.x] = static_cast<unsigned>(min(total, 0xFFFFFFFFull));
+    unsigned total;
+    block_excl_scan<kScanThreads>(v, s_tmp, total);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
 // Ranges, first free positions (cursor) and, for lists of more than kTileChunk pairs, the list of
@@ -95,12 +67,18 @@ __global__ void __launch_bounds__(kScanThreads) tile_scan_kernel(const unsigned*
                                                                  uint2* __restrict__ chunks, unsigned chunk_cap,
                                                                  unsigned capacity, Ctrl* ctrl) {
     chain_entry();
-    __shared__ unsigned long long s_tmp[kScanThreads / 32];
+    __shared__ unsigned s_tmp[kScanThreads / 32];
     const unsigned long long t0 = static_cast<unsigned long long>(blockIdx.x) * kScanTiles + threadIdx.x * kScanPer;
-    unsigned cnt[kScanPer];
-    unsigned long long own = 0, before = 0;
+    // The preprocess's total counts whole rectangles, so the pairs to sort are at most as many, and
+    // within the capacity every sum fits 32 bits.
+    const bool over = ctrl->pair_total > capacity;
+    unsigned cnt[kScanPer], own = 0, before = 0;
 #pragma unroll
     for (int k = 0; k < kScanPer; ++k) cnt[k] = t0 + k < tiles ? counts[(t0 + k) * kTileStride] : 0u;
+    if (over) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&ctrl->flags, kFlagOverflow);
+        return;
+    }
     if (sums) {
         for (unsigned b = threadIdx.x; b < blockIdx.x; b += kScanThreads) before += sums[b];
     } else {
@@ -110,17 +88,12 @@ __global__ void __launch_bounds__(kScanThreads) tile_scan_kernel(const unsigned*
     }
 #pragma unroll
     for (int k = 0; k < kScanPer; ++k) own += cnt[k];
-    unsigned long long all;
+    unsigned all;
     if (blockIdx.x) {
-        scan_u64(before, s_tmp, all);
+        block_excl_scan<kScanThreads>(before, s_tmp, all);
         before = all;
     }
-    const unsigned long long ex = scan_u64(own, s_tmp, all);
-    // The preprocess's total counts whole rectangles, so the pairs to sort are at most as many.
-    const bool over = ctrl->pair_total > capacity;
-    if (over && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&ctrl->flags, kFlagOverflow);
-    if (over) return;
-    unsigned start = static_cast<unsigned>(before + ex);
+    unsigned start = before + block_excl_scan<kScanThreads>(own, s_tmp, all);
 #pragma unroll
     for (int k = 0; k < kScanPer; ++k) {
         if (t0 + k >= tiles) break;
@@ -139,10 +112,10 @@ __global__ void __launch_bounds__(kScanThreads) tile_scan_kernel(const unsigned*
 // ---- scatter -------------------------------------------------------------------------------------
 
 constexpr unsigned kScatterEntries = kThreads;  // entries per CTA and round
-constexpr int kScatterPairs = 4;                               // pairs per lane whose atomics are in flight together
+constexpr unsigned kFewEntries = 1u << 21;  // up to here a warp keeps four pairs per lane in flight, above it two
 constexpr unsigned kLargeArea = 1024;  // an entry of more tiles is left to the whole CTA
 
-// Appends pair k of the rectangle (w tiles wide, corner tile org, tx tiles per row of its view).
+// Tile k of a rectangle w tiles wide with corner tile org, in a view of tx tiles per row.
 __device__ __forceinline__ unsigned tile_of(unsigned k, unsigned org, unsigned w, unsigned tx) {
     const unsigned row = k / w;
     return org + row * tx + (k - row * w);
@@ -153,6 +126,13 @@ __device__ __forceinline__ unsigned tile_of(unsigned k, unsigned org, unsigned w
 // holds kScatterPairs appends in flight whatever the rectangles' sizes; entries of more than
 // kLargeArea tiles go to the whole CTA afterwards. offs (training; else NULL) receives each
 // entry's first gradient slot, allocated per CTA and round in any order.
+// kScatterPairs: four where the frame is short of warps and waits for the adds, two in a large frame,
+// whose instructions count (a warp's 32 entries have 43 to 69 pairs in the views measured): 191 against
+// 193 us per 740k frame, but 6.25 against 6.00 ms for the 64-view batch; equal at 2.2M entries.
+// (Spreading the pairs of a CTA's 256 to 1024 entries over its threads takes a fifth of the instructions
+// and is no faster; nor is ranking small entries' pairs as they are counted, which saves the scatter
+// four fifths of its adds: the scattered accesses themselves bound it.)
+template <int kScatterPairs>
 __global__ void __launch_bounds__(kThreads) tile_scatter_kernel(const unsigned* __restrict__ depth_key,
                                                                 const unsigned long long* __restrict__ rect16,
                                                                 unsigned entries, BatchTables tables,
@@ -570,7 +550,8 @@ void launch_tile_sort(const TileSortArgs& a, cudaStream_t stream) {
                    sums ? static_cast<const unsigned*>(a.sums) : nullptr, a.ranges, a.cursor, a.chunks, a.chunk_cap,
                    a.capacity, a.ctrl);
     const unsigned rounds = static_cast<unsigned>((static_cast<uint64_t>(a.entries) + kScatterEntries - 1) / kScatterEntries);
-    launch_chained(tile_scatter_kernel, dim3(std::max(1u, std::min(rounds, 148u * 32u))), dim3(kThreads), stream,
+    const auto scatter = a.entries <= kFewEntries ? tile_scatter_kernel<4> : tile_scatter_kernel<2>;
+    launch_chained(scatter, dim3(std::max(1u, std::min(rounds, 148u * 32u))), dim3(kThreads), stream,
                    a.depth_key, a.rect16, a.entries, a.tables, a.cursor, a.pairs, a.offs, a.ctrl);
     const unsigned further = std::min(a.chunk_cap, 296u);
     launch_chained(tile_sort_kernel, dim3(a.tiles + further), dim3(kThreads), stream, a.ranges, a.tiles, a.chunks,
