@@ -41,6 +41,7 @@ struct CamParams {
 };
 
 struct SceneView {
+    static constexpr bool kCrossXz = true;  // rounding of the covariance (covariance() of the preprocess)
     const float4* pos_op;
     const float4* scale;
     const float4* rot;
@@ -61,6 +62,7 @@ struct SceneView {
 // of 4 (sh_planes = 3K / 4). Activated on the fly as the reference loader activates a PLY
 // (ply_loader.cpp:124-131): exp, sigmoid, normalise.
 struct RawParams {
+    static constexpr bool kCrossXz = false;
     const float* means;
     const float* log_scales;
     const float4* quats;

@@ -102,18 +102,29 @@ struct Cov3 {
     }
 };
 
+// The rotation's products each occur in two sums, so which of a sum's two products the compiler rounds
+// before it fuses the other depends on the code around it. The choice is written out here, so that every
+// instantiation of the kernel gives a splat the same bits: kCrossXz (of the scene's layout) says whether
+// x z or w y is the rounded product of the two sums that hold both.
+template <bool kCrossXz>
 __device__ __forceinline__ void covariance(const float4 sg, const float4 q, float splat_scale, Cov3& o) {
     const float w = q.x, x = q.y, y = q.z, z = q.w;
-    const float Rq[3][3] = {{1 - 2 * (y * y + z * z), 2 * (x * y - w * z), 2 * (x * z + w * y)},
-                            {2 * (x * y + w * z), 1 - 2 * (x * x + z * z), 2 * (y * z - w * x)},
-                            {2 * (x * z - w * y), 2 * (y * z + w * x), 1 - 2 * (x * x + y * y)}};
+    const float wx = __fmul_rn(w, x), wy = __fmul_rn(w, y), wz = __fmul_rn(w, z), xz = __fmul_rn(x, z);
+    const float yy = __fmul_rn(y, y), zz = __fmul_rn(z, z);
+    const float xz_plus = kCrossXz ? __fmaf_rn(w, y, xz) : __fmaf_rn(x, z, wy);
+    const float xz_minus = kCrossXz ? __fmaf_rn(-w, y, xz) : __fmaf_rn(x, z, -wy);
+    const float Rq[3][3] = {{1 - 2 * __fadd_rn(yy, zz), 2 * __fmaf_rn(x, y, -wz), 2 * xz_plus},
+                            {2 * __fmaf_rn(x, y, wz), 1 - 2 * __fmaf_rn(x, x, zz), 2 * __fmaf_rn(y, z, -wx)},
+                            {2 * xz_minus, 2 * __fmaf_rn(y, z, wx), 1 - 2 * __fmaf_rn(x, x, yy)}};
     const float s[3] = {sg.x * splat_scale, sg.y * splat_scale, sg.z * splat_scale};
     float M[3][3];
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) M[r][c] = Rq[r][c] * s[c];
-    const auto dot = [&](int r, int c) { return M[r][0] * M[c][0] + M[r][1] * M[c][1] + M[r][2] * M[c][2]; };
+        for (int c = 0; c < 3; ++c) M[r][c] = __fmul_rn(Rq[r][c], s[c]);
+    const auto dot = [&](int r, int c) {
+        return __fmaf_rn(M[r][2], M[c][2], __fmaf_rn(M[r][0], M[c][0], __fmul_rn(M[r][1], M[c][1])));
+    };
     o.s00 = dot(0, 0);
     o.s01 = dot(0, 1);
     o.s02 = dot(0, 2);
@@ -440,7 +451,7 @@ __global__ void __launch_bounds__(kPreThreads, 8) preprocess_kernel(const BatchS
 #pragma unroll
         for (int g = 0; g < kPreGroups; ++g) {
             Cov3 cov;
-            covariance(sg[g], q[g], scale, cov);
+            covariance<Src::kCrossXz>(sg[g], q[g], scale, cov);
             s_pos[g * kPreThreads + tid] = pg[g];
             s_cova[g * kPreThreads + tid] = make_float4(cov.s00, cov.s01, cov.s02, cov.s11);
             s_covb[g * kPreThreads + tid] = make_float4(cov.s12, cov.s22, cov.trace, scale);
@@ -454,7 +465,7 @@ __global__ void __launch_bounds__(kPreThreads, 8) preprocess_kernel(const BatchS
         if (cam.splatScale != cb.w) {
             float4 pg2, sg, q;
             sc.src.load(block_first + slot, pg2, sg, q);
-            covariance(sg, q, cam.splatScale, cov);
+            covariance<Src::kCrossXz>(sg, q, cam.splatScale, cov);
         }
         return cov;
     };
