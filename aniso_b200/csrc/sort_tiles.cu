@@ -412,7 +412,12 @@ __device__ __forceinline__ void sort_chunk(const unsigned long long* src, unsign
 
 // CTA b < tiles sorts tile b's first chunk, the others take the further chunks of long lists in turn.
 // A list of one chunk is written as sorted entries; a chunk of a longer one goes back in place.
-__global__ void __launch_bounds__(kThreads) tile_sort_kernel(const uint2* __restrict__ ranges, unsigned tiles,
+// Latency-bound: eight CTAs per SM (32 registers, where only the merge sort spills) instead of five take
+// 192 to 189 us off the 740k frame, 403 to 396 us at 2.2M / 1920x1080, 2.29 to 2.22 ms off 16 views. Crowded
+// depths (the merge sort) cost little: a wall of 740k splats takes 271 us a frame, a plane 277 us (with the
+// LSD chain 365 and 503 us). Chunks of 1024 in CTAs of 128 threads: 392 us and 2.19 ms, but the lists of
+// small images then need merging (the 64-view batch 6.15 against 5.92 ms).
+__global__ void __launch_bounds__(kThreads, 8) tile_sort_kernel(const uint2* __restrict__ ranges, unsigned tiles,
                                                              const uint2* __restrict__ chunks, unsigned chunk_cap,
                                                              unsigned long long* pairs,
                                                              unsigned* __restrict__ vals, const Ctrl* ctrl) {
