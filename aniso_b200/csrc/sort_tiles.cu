@@ -410,6 +410,28 @@ __device__ __forceinline__ void sort_chunk(const unsigned long long* src, unsign
     }
 }
 
+// One warp's sort of n (0..kShortList) pairs at src into entries at out, two pairs per lane: a pair's place
+// is the number of smaller ones, counted as the warp passes every pair round.
+constexpr unsigned kShortList = 64;
+constexpr unsigned kSparseEntries = 32;  // entries (visible or not) per tile below which a frame is sparse
+__device__ __forceinline__ void sort_short(const unsigned long long* src, unsigned n, unsigned* out) {
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned long long x0 = lane < n ? src[lane] : kNoPair, x1 = lane + 32 < n ? src[lane + 32] : kNoPair;
+    unsigned place0 = 0, place1 = 0;
+    for (unsigned j = 0; j < min(n, 32u); ++j) {
+        const unsigned long long x = __shfl_sync(0xFFFFFFFFu, x0, j);
+        place0 += x < x0;
+        place1 += x < x1;
+    }
+    for (unsigned j = 32; j < n; ++j) {
+        const unsigned long long x = __shfl_sync(0xFFFFFFFFu, x1, j - 32);
+        place0 += x < x0;
+        place1 += x < x1;
+    }
+    if (lane < n) out[place0] = static_cast<unsigned>(x0);
+    if (lane + 32 < n) out[place1] = static_cast<unsigned>(x1);
+}
+
 // CTA b < tiles sorts tile b's first chunk, the others take the further chunks of long lists in turn.
 // A list of one chunk is written as sorted entries; a chunk of a longer one goes back in place.
 // Latency-bound: eight CTAs per SM (32 registers, where only the merge sort spills) instead of five take
@@ -417,6 +439,14 @@ __device__ __forceinline__ void sort_chunk(const unsigned long long* src, unsign
 // depths (the merge sort) cost little: a wall of 740k splats takes 271 us a frame, a plane 277 us (with the
 // LSD chain 365 and 503 us). Chunks of 1024 in CTAs of 128 threads: 392 us and 2.19 ms, but the lists of
 // small images then need merging (the 64-view batch 6.15 against 5.92 ms).
+//
+// A list of at most kShortList pairs is sorted by one warp. Where a frame has few entries for its tiles
+// (kSparse), most lists are that short or empty, and a CTA takes eight tiles, a warp each, and then their
+// longer lists one after another: ten 572x327 views of
+// 32k Gaussians in 8x8 tiles take 295 us a frame with a CTA's sort for every list, 238 with the warp's,
+// 214 with eight tiles per CTA; four 1660x984 views of two scenes of 20k in 16x32 tiles 269, 242, 230 us.
+// With many entries per tile a CTA per tile is the better one: 2.22 against 2.24 ms for 16 views of 740k.
+template <bool kSparse>
 __global__ void __launch_bounds__(kThreads, 8) tile_sort_kernel(const uint2* __restrict__ ranges, unsigned tiles,
                                                              const uint2* __restrict__ chunks, unsigned chunk_cap,
                                                              unsigned long long* pairs,
@@ -424,18 +454,38 @@ __global__ void __launch_bounds__(kThreads, 8) tile_sort_kernel(const uint2* __r
     chain_entry();
     __shared__ SortShared sh;
     if (ctrl->flags & kFlagOverflow) return;
-    if (blockIdx.x < tiles) {
-        const uint2 r = ranges[blockIdx.x];
-        const unsigned n = r.y - r.x;
-        if (n == 0) return;
-        if (n <= kTileChunk)
-            sort_chunk(pairs + r.x, n, sh, [&](unsigned i, unsigned long long x) { vals[r.x + i] = static_cast<unsigned>(x); });
-        else
-            sort_chunk(pairs + r.x, kTileChunk, sh, [&](unsigned i, unsigned long long x) { pairs[r.x + i] = x; });
+    constexpr unsigned kTiles = kSparse ? kWarps : 1;  // of a CTA
+    const unsigned list_ctas = (tiles + kTiles - 1) / kTiles;
+    if (blockIdx.x < list_ctas) {
+        const auto sort_list = [&](uint2 r, unsigned n) {
+            if (n <= kTileChunk)
+                sort_chunk(pairs + r.x, n, sh, [&](unsigned i, unsigned long long x) { vals[r.x + i] = static_cast<unsigned>(x); });
+            else
+                sort_chunk(pairs + r.x, kTileChunk, sh, [&](unsigned i, unsigned long long x) { pairs[r.x + i] = x; });
+        };
+        if (!kSparse) {
+            const uint2 r = ranges[blockIdx.x];
+            const unsigned n = r.y - r.x;
+            if (n > kShortList) sort_list(r, n);
+            else if (threadIdx.x < 32) sort_short(pairs + r.x, n, vals + r.x);
+            return;
+        }
+        const unsigned first = blockIdx.x * kTiles, end = min(first + kTiles, tiles), mine = first + (threadIdx.x >> 5);
+        if (mine < end) {
+            const uint2 r = ranges[mine];
+            if (r.y - r.x <= kShortList) sort_short(pairs + r.x, r.y - r.x, vals + r.x);
+        }
+        for (unsigned t = first; t < end; ++t) {
+            const uint2 r = ranges[t];
+            const unsigned n = r.y - r.x;
+            if (n <= kShortList) continue;
+            __syncthreads();
+            sort_list(r, n);
+        }
         return;
     }
     const unsigned count = min(ctrl->chunk_count, chunk_cap);
-    for (unsigned c = blockIdx.x - tiles; c < count; c += gridDim.x - tiles) {
+    for (unsigned c = blockIdx.x - list_ctas; c < count; c += gridDim.x - list_ctas) {
         const uint2 ch = chunks[c];
         if (ch.y == 0) continue;
         const uint2 r = ranges[ch.x];
@@ -559,8 +609,10 @@ void launch_tile_sort(const TileSortArgs& a, cudaStream_t stream) {
     launch_chained(scatter, dim3(std::max(1u, std::min(rounds, 148u * 32u))), dim3(kThreads), stream,
                    a.depth_key, a.rect16, a.entries, a.tables, a.cursor, a.pairs, a.offs, a.ctrl);
     const unsigned further = std::min(a.chunk_cap, 296u);
-    launch_chained(tile_sort_kernel, dim3(a.tiles + further), dim3(kThreads), stream, a.ranges, a.tiles, a.chunks,
-                   a.chunk_cap, a.pairs, a.vals, a.ctrl);
+    const bool sparse = a.entries / kSparseEntries < a.tiles;
+    const unsigned list_ctas = sparse ? (a.tiles + kWarps - 1) / kWarps : a.tiles;
+    launch_chained(sparse ? tile_sort_kernel<true> : tile_sort_kernel<false>, dim3(list_ctas + further), dim3(kThreads),
+                   stream, a.ranges, a.tiles, a.chunks, a.chunk_cap, a.pairs, a.vals, a.ctrl);
     if (a.longest <= kTileChunk) return;
     launch_chained(tile_merge_kernel, dim3(std::min(a.chunk_cap, 592u)), dim3(kThreads), stream, a.ranges, a.chunks,
                    a.chunk_cap, a.pairs, a.merged, a.vals, a.ctrl);
