@@ -336,10 +336,10 @@ void enqueue_tile_sort(Arena& A, unsigned entries, unsigned longest, unsigned ti
 // that count matrix first; every other pass has its own upsweep. (Counting in the downsweeps too
 // was measured slower: keys written next to each other often share the next digit, the high depth
 // digits taking few values, so one atomic per key contends -- 0.177 ms against 0.139 ms for the
-// sort of the 740k / 1280x720 frame.) A frame of at most bin_max_tiles() tiles (A.bins_for) takes
+// sort of the 740k / 1280x720 frame, when this chain sorted it.) A frame of at most bin_max_tiles() tiles (A.bins_for) takes
 // the one-pass tile binning after the expansion instead of the tile passes and the ranges.
 // short_depth: every visible key is below 2^27 (Plan::bound_depth), so three 9-bit depth passes
-// replace the four 8-bit ones (measured 0.119 -> 0.111 ms of sort for the 740k frame). Where the
+// replace the four 8-bit ones (0.119 -> 0.111 ms of sort for the 740k frame, when this chain sorted it). Where the
 // persistent sort is selected (A.ctas), it replaces this whole sequence with one launch and the
 // same outputs.
 int enqueue_sort(Arena& A, unsigned entries, unsigned tiles, const BatchTables& tables, bool keep_rank, int bits,
@@ -563,7 +563,8 @@ struct Plan {
 
     // Picks the short depth passes when every view's scene box (boxes[s], NULL: unknown) keeps its
     // depths below 8192 for the view's camera, and the frame has at most kProducerCountMax entries
-    // (larger frames' 9-bit passes were measured slower: the 64-view 1M batch 8.69 -> 8.75 ms).
+    // (larger frames' 9-bit passes were measured slower: the 64-view 1M batch 8.69 -> 8.75 ms when the LSD
+    // chain sorted it).
     // Without a call (the training path's positions change every step) the frame keeps 8-bit passes.
     void bound_depth(const std::vector<const PositionBox*>& boxes) {
         short_depth = entries > 0 && entries <= kProducerCountMax;

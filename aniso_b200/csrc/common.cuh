@@ -219,7 +219,7 @@ __device__ __forceinline__ void count_key(const PassCounts& pc, unsigned blocks,
 }
 
 // ---- programmatic dependent launch --------------------------------------------------------------
-// The frame is a chain of ~25 dependent kernels, most of them a few microseconds long, so the gap
+// The frame is a chain of dependent kernels, many of them a few microseconds long, so the gap
 // between one kernel's end and the next kernel's start (grid completion, memory flush, launch,
 // CTA dispatch) is a visible share of the frame. Kernels of the chain are launched with
 // programmatic stream serialisation (launch_chained), which lets the next launch be prepared while

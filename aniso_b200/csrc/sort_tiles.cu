@@ -444,7 +444,7 @@ __device__ __forceinline__ void sort_short(const unsigned long long* src, unsign
 // (kSparse), most lists are that short or empty, and a CTA takes eight tiles, a warp each, and then their
 // longer lists one after another: ten 572x327 views of
 // 32k Gaussians in 8x8 tiles take 295 us a frame with a CTA's sort for every list, 238 with the warp's,
-// 214 with eight tiles per CTA; four 1660x984 views of two scenes of 20k in 16x32 tiles 269, 242, 230 us.
+// 214 with eight tiles per CTA; eight 1660x984 views of two scenes of 20k in 16x32 tiles 269, 242, 230 us.
 // With many entries per tile a CTA per tile is the better one: 2.22 against 2.24 ms for 16 views of 740k.
 template <bool kSparse>
 __global__ void __launch_bounds__(kThreads, 8) tile_sort_kernel(const uint2* __restrict__ ranges, unsigned tiles,
