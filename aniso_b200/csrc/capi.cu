@@ -591,7 +591,9 @@ struct Plan {
         return (b + 15) / 16 * 16;
     }
     size_t blob_bytes() const { return grads_offset() + grads.size() * sizeof(RawGrads); }
-    // Same launch geometry (the only thing a recorded graph fixes besides the slot).
+    // Same launch geometry (the only thing a recorded graph fixes besides the slot). Which scene each view
+    // shows is part of it: the adjoint's launches name the view's scene and size, and the longest list a
+    // tile can have decides which merge kernels the sort has.
     bool same_geometry(const Plan& o) const {
         if (views.size() != o.views.size() || scenes.size() != o.scenes.size() || entries != o.entries ||
             tiles != o.tiles || grads.size() != o.grads.size() || pre_blocks != o.pre_blocks ||
@@ -600,8 +602,8 @@ struct Plan {
         for (size_t s = 0; s < scenes.size(); ++s)
             if (scenes[s].src.n != o.scenes[s].src.n) return false;
         for (size_t k = 0; k < views.size(); ++k)
-            if (views[k].cam.width != o.views[k].cam.width || views[k].cam.height != o.views[k].cam.height ||
-                views[k].cam.shDegree != o.views[k].cam.shDegree)
+            if (views[k].scene != o.views[k].scene || views[k].cam.width != o.views[k].cam.width ||
+                views[k].cam.height != o.views[k].cam.height || views[k].cam.shDegree != o.views[k].cam.shDegree)
                 return false;
         return shape.tile_w == o.shape.tile_w && shape.tile_h == o.shape.tile_h &&
                shape.blend_batch == o.shape.blend_batch && shape.radix_bits == o.shape.radix_bits &&
