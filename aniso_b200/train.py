@@ -174,12 +174,13 @@ class _LossFunction(torch.autograd.Function):
 
 def _loss(img: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
     """0.8 L1 + 0.2 (1 - SSIM) (train_gsplat.py:178-180). The library's two kernels take float32 CUDA
-    images of one shape, 11 pixels a side at least (the window), with a constant target, and
+    images of one shape (H, W, 3), 11 (the window) to 32767 pixels a side, with a constant target, and
     give the composed expression's gradient bit for bit (2.6 ms of a 1280x720 step became 0.23 ms).
-    Anything else (a differentiable target, say) is composed from torch
-    operations."""
+    Anything else (a differentiable target, say) is composed from torch operations, which raise for
+    images of another rank or channel count."""
     if (img.is_cuda and target.is_cuda and img.device == target.device and img.dtype == target.dtype == torch.float32
-            and img.shape == target.shape and min(img.shape[:2]) >= 11 and not target.requires_grad):
+            and img.shape == target.shape and img.dim() == 3 and img.shape[2] == 3 and min(img.shape[:2]) >= 11
+            and max(img.shape[:2]) <= 32767 and not target.requires_grad):
         return _LossFunction.apply(img, target, 0.8, 0.2)
     return 0.8 * (img - target).abs().mean() + 0.2 * (1 - ssim(img, target))
 
