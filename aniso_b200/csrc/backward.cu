@@ -16,6 +16,10 @@
 //   the sums' shared memory leaves. Measured at 2.2M / 1280x720: 647 us with one list per warp and
 //   warp-wide shuffles, 587 us with lists per quarter, 569 us with the sums through shared memory and
 //   room for 512 of them (6 CTAs per SM; 640 and 768: 585 us).
+//   Sparse frames (sparse_frame) take rounds of 32 splats, whose masks and lists are one ballot each, and leave
+//   empty tiles at once; 16x32 tiles are held to 85 registers for three CTAs instead of two. Forward and
+//   backward of twelve 1600x900 views of three scenes of 10k to 20k: 1279 -> 1050 us in 16x32 tiles, 1102 -> 999
+//   in 16x16 (with one list per warp 1115, 1010); of twelve 640x360 views of 200k to 400k, 16x32: 1724 -> 1664.
 // gauss_backward: one launch per view over the Gaussians visible in it (compacted first, so no lane
 //   idles on a culled one); each sums its pairs' slots (contiguous, in a fixed order), applies the
 //   chain rule through the record
@@ -32,7 +36,7 @@
 namespace ab2 {
 namespace {
 
-constexpr int kBatch = 128;
+constexpr int kBackwardBatch = 128, kBackwardSparseBatch = 32;  // splats of a round, and in a sparse frame
 constexpr int kBackwardPlaces = 512;  // (splat, cell) sums a 16x16 tile's round has room for
 constexpr int kG = 9;
 constexpr float kLn2 = 0.69314718055994530942f;
@@ -121,10 +125,11 @@ constexpr int kRedPitch = 36;  // floats per value: a quarter's eight lanes as t
 // Shared memory of one CTA. A quarter warp's sums for the splats of its list go to consecutive places
 // of grad; at[slot][list] is where a staged splat's sums of that list start (place kPlaces, which holds
 // zeros, where the list leaves the splat out).
-template <int TW, int TH>
+template <int TW, int TH, int kBatch>
 struct BackwardShared {
     static constexpr int kLists = TW * TH / 16;           // quarter warps: cells of 2 x 8 pixels
-    static constexpr int kPlaces = TW * TH == 64 ? 4 * kBatch : TW * TH * kBackwardPlaces / 256;
+    static constexpr int kRoom = TW * TH * kBackwardPlaces / 256;
+    static constexpr int kPlaces = TW * TH == 64 || kBatch * kLists < kRoom ? kBatch * kLists : kRoom;
     float4 r0[kBatch + 1];                                // the last slot: a splat that no pixel takes
     float4 r1[kBatch + 1];
     unsigned short at[kBatch][kLists];
@@ -142,14 +147,14 @@ struct BackwardShared {
 // the row), so that the sum over a splat's pixels -- rows by shuffles within the quarter, then the
 // quarters as (0 + 2) + (1 + 3), then the warps in order -- runs in a fixed order whichever quarters a
 // splat reaches.
-template <int TW, int TH>
-__global__ void __launch_bounds__(TW * TH / 2) blend_backward_kernel(BackwardIn in, float* __restrict__ grad_pair) {
+template <int TW, int TH, int kBatch>
+__global__ void __launch_bounds__(TW * TH / 2, TW * TH == 512 ? 3 : 0) blend_backward_kernel(BackwardIn in, float* __restrict__ grad_pair) {
     chain_entry();
     constexpr int kThreads = TW * TH / 2;
     constexpr int kWarps = kThreads / 32;
     constexpr int kWarpsX = TW / 8;
     constexpr int kCells = TW / 2;  // cells per 8-row band of the tile
-    using Shared = BackwardShared<TW, TH>;
+    using Shared = BackwardShared<TW, TH, kBatch>;
     constexpr unsigned kPlaces = Shared::kPlaces;
     extern __shared__ __align__(16) unsigned char s_raw[];
     Shared& sh = *reinterpret_cast<Shared*>(s_raw);
@@ -165,6 +170,7 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_backward_kernel(BackwardIn 
     const int width = vi.cam.width, height = vi.cam.height;
     const float px0 = x0 + 0.5f, py = y + 0.5f;
     const uint2 range = (in.ctrl->flags & kFlagOverflow) ? make_uint2(0, 0) : in.ranges[gtile];
+    if (kBatch == kBackwardSparseBatch && range.x == range.y) return;
     const int cell0 = (warp / kWarpsX) * kCells + (warp % kWarpsX) * 4;  // the warp's first cell in a mask
     const int sumq = lane & 3, sumk = lane >> 2;  // the quarter and value whose eight lanes this lane sums
 
@@ -189,8 +195,8 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_backward_kernel(BackwardIn 
         st.gb.y = vi.grad_img[3 * p + 2];
     }
     // An infinite or NaN gradient times a weight of zero is NaN: where the warp holds one, a lane whose
-    // pixels a splat does not apply to adds zeros to its sums all the same, in a walk of its own (selects in
-    // the one walk cost the 2.2M view 1%).
+    // pixels a splat does not apply to adds zeros to its sums all the same, in a walk of its own (496 -> 502 us
+    // of adjoint blend at 2.2M / 1280x720; with the selects in the one walk 508).
     const bool hostile = __any_sync(0xFFFFFFFFu, !isfinite(st.gr.x + st.gg.x + st.gb.x + st.gr.y + st.gg.y + st.gb.y));
     if (tid == 0) {
         sh.maxlast = range.x;
@@ -330,9 +336,9 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_backward_kernel(BackwardIn 
                 if (__any_sync(0xFFFFFFFFu, test.v0 || test.v1)) {  // else the sums are zero
                     float g[kG];
                     pixel_step2(st, test, dx, dy, r0, r1, rb, g);
-                    if (decltype(guarded)::value)
+                    if (decltype(guarded)::value)  // the colour sums: the others are selected to zero already
 #pragma unroll
-                        for (int k = 0; k < kG; ++k) g[k] = test.v0 || test.v1 ? g[k] : 0.f;
+                        for (int k = 6; k < kG; ++k) g[k] = test.v0 || test.v1 ? g[k] : 0.f;
 #pragma unroll
                     for (int k = 0; k < 8; ++k) red[k * kRedPitch] = g[k];
                     ninth = g[8];
@@ -763,28 +769,36 @@ __global__ void __launch_bounds__(128, 4) gauss_backward_kernel(const BatchScene
 }  // namespace
 
 namespace {
-template <int TW, int TH>
+template <int TW, int TH, int kBatch>
 void launch_blend_backward_t(const BackwardIn& in, unsigned tiles, float* grad_pair, cudaStream_t stream) {
     constexpr int kDevices = 64;
+    constexpr size_t kShared = sizeof(BackwardShared<TW, TH, kBatch>);
     static std::atomic<bool> raised[kDevices];  // the dynamic shared memory limit, once per device
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kDevices && !raised[dev]) {
-        if (cudaFuncSetAttribute(blend_backward_kernel<TW, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(sizeof(BackwardShared<TW, TH>))) == cudaSuccess)
+        if (cudaFuncSetAttribute(blend_backward_kernel<TW, TH, kBatch>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(kShared)) == cudaSuccess)
             raised[dev] = true;
     }
     cudaGetLastError();  // a failed raise shows up as the launch's error
-    launch_chained_smem(blend_backward_kernel<TW, TH>, dim3(tiles), dim3(TW * TH / 2), sizeof(BackwardShared<TW, TH>),
-                        stream, in, grad_pair);
+    launch_chained_smem(blend_backward_kernel<TW, TH, kBatch>, dim3(tiles), dim3(TW * TH / 2), kShared, stream, in,
+                        grad_pair);
+}
+
+template <int kBatch>
+void launch_blend_backward_rounds(const BackwardIn& in, unsigned tiles, int tile_w, int tile_h, float* grad_pair,
+                                  cudaStream_t stream) {
+    if (tile_w == 8) launch_blend_backward_t<8, 8, kBatch>(in, tiles, grad_pair, stream);
+    else if (tile_h == 32) launch_blend_backward_t<16, 32, kBatch>(in, tiles, grad_pair, stream);
+    else launch_blend_backward_t<16, 16, kBatch>(in, tiles, grad_pair, stream);
 }
 }  // namespace
 
-void launch_blend_backward(const BackwardIn& in, unsigned tiles, int tile_w, int tile_h, float* grad_pair,
+void launch_blend_backward(const BackwardIn& in, unsigned tiles, int tile_w, int tile_h, bool sparse, float* grad_pair,
                            cudaStream_t stream) {
     if (tiles == 0) return;
-    if (tile_w == 8) launch_blend_backward_t<8, 8>(in, tiles, grad_pair, stream);
-    else if (tile_h == 32) launch_blend_backward_t<16, 32>(in, tiles, grad_pair, stream);
-    else launch_blend_backward_t<16, 16>(in, tiles, grad_pair, stream);
+    if (sparse) launch_blend_backward_rounds<kBackwardSparseBatch>(in, tiles, tile_w, tile_h, grad_pair, stream);
+    else launch_blend_backward_rounds<kBackwardBatch>(in, tiles, tile_w, tile_h, grad_pair, stream);
 }
 
 namespace {

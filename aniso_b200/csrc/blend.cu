@@ -29,6 +29,13 @@
 //   * a finished pixel holds T = 0 (T >= 1e-4 while it is not finished), so no separate flag is
 //     carried; the warp leaves once all 64 pixels are finished and the block stops loading once all
 //     its warps have (__syncthreads_or).
+//   * a sparse frame (sparse_frame: under 32 entries per tile) is bound by the latency of each tile's few
+//     splats, not by issue: the ellipse test, the lists and their padding took longer than the steps they
+//     saved, and 56 to 85 registers and 19 KB left room for fewer CTAs. It takes instantiations of their own:
+//     rounds of 128 (16x32: 256) splats, cells by the bounds alone, no lists where a round holds at most
+//     32 splats, empty tiles left at once, 48 registers (16x16, 16x32). Eight 1660x984 views of two scenes of
+//     20k: 410 -> 258 us a batch in 8x8 tiles, 239 -> 192 in 16x16, 236 -> 186 in 16x32 (with one list per warp
+//     333, 228, 234).
 // Tried and slower: comparisons as 0 / 1 floats with packed products in place of the selects
 // (+1.5% per frame), predicated scalar updates (+4%), operands staged in pairs (+5.5%), ten CTAs per
 // SM by holding the kernel to 48 registers (+3%).
@@ -94,8 +101,8 @@ __device__ __forceinline__ unsigned quantise(float c) {
 // else 4-byte ones, else single bytes. Wide contiguous stores matter most when `out` is pinned
 // host memory written across PCIe during the blend (each store instruction becomes a few bus
 // writes, where per-pixel bytes would become many partial ones); in device memory they cost no
-// more than per-pixel stores.
-template <int TW, int TH, int kThreads>
+// more than per-pixel stores. kBlack: zeros, nothing is read.
+template <int TW, int TH, int kThreads, bool kBlack = false>
 __device__ __forceinline__ void write_tile_rgb8(const unsigned char* s_px, uint8_t* out, int width, int height,
                                                 int ox, int oy) {
     constexpr int kRow = TW * 3;
@@ -108,25 +115,25 @@ __device__ __forceinline__ void write_tile_rgb8(const unsigned char* s_px, uint8
         for (int i = threadIdx.x; i < rows * per; i += kThreads) {
             const int r = i / per, c = i - r * per;
             *reinterpret_cast<uint4*>(dst + r * pitch + c * 16) =
-                *reinterpret_cast<const uint4*>(s_px + r * kRow + c * 16);
+                kBlack ? make_uint4(0, 0, 0, 0) : *reinterpret_cast<const uint4*>(s_px + r * kRow + c * 16);
         }
     } else if ((a & 3) == 0) {
         const int per = seg >> 2;
         for (int i = threadIdx.x; i < rows * per; i += kThreads) {
             const int r = i / per, c = i - r * per;
             *reinterpret_cast<unsigned*>(dst + r * pitch + c * 4) =
-                *reinterpret_cast<const unsigned*>(s_px + r * kRow + c * 4);
+                kBlack ? 0u : *reinterpret_cast<const unsigned*>(s_px + r * kRow + c * 4);
         }
     } else {
         for (int i = threadIdx.x; i < rows * seg; i += kThreads) {
             const int r = i / seg, c = i - r * seg;
-            dst[r * pitch + c] = s_px[r * kRow + c];
+            dst[r * pitch + c] = kBlack ? static_cast<unsigned char>(0) : s_px[r * kRow + c];
         }
     }
 }
 
-template <int TW, int TH, int kBatch, bool kTrain>
-__global__ void __launch_bounds__(TW * TH / 2) blend_kernel(const uint2* __restrict__ ranges,
+template <int TW, int TH, int kBatch, bool kTrain, bool kSparse>
+__global__ void __launch_bounds__(TW * TH / 2, kSparse ? 1280 / (TW * TH / 2) : 0) blend_kernel(const uint2* __restrict__ ranges,
                                                             const unsigned* __restrict__ vals,
                                                             const SplatRecord* __restrict__ rec, const Ctrl* ctrl,
                                                             const ViewInfo* __restrict__ views, BatchTables tables) {
@@ -157,6 +164,14 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_kernel(const uint2* __restr
     // The warp's cells in a staged splat's mask: quarters 0 and 1 at this bit, 2 and 3 one row below.
     const int cell0 = (warp / kWarpsX) * 2 * kCells + (warp % kWarpsX) * 2;
 
+    if (kSparse && range.x == range.y) {  // an empty tile
+        if (kTrain) {
+            store_train_px(vi, x0, y, 1.0f, 0.f, 0.f, 0.f, range.x);
+            store_train_px(vi, x0 + 1, y, 1.0f, 0.f, 0.f, 0.f, range.x);
+        }
+        if (vi.rgb8) write_tile_rgb8<TW, TH, kThreads, true>(nullptr, vi.rgb8, width, height, ox, oy);
+        return;
+    }
     if (tid == 0) {
         s_r0[kBatch] = make_float4(0.f, 0.f, 0.f, 0.f);
         s_r1[kBatch] = make_float4(0.f, -INFINITY, 0.f, 0.f);
@@ -182,7 +197,7 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_kernel(const uint2* __restr
                 s_r0[slot] = r.r0;
                 s_r1[slot] = make_float4(r.r1.x, r.r1.y, fminf(r.r1.z, kMax), fminf(r.r1.w, kMax));
                 s_b[slot] = fminf(r.r2.x, kMax);
-                m = staged_cell_mask<TW, TH, 4, 4>(r, ox, oy);
+                m = staged_cell_mask<TW, TH, 4, 4, !kSparse>(r, ox, oy);
             }
             s_mask[slot] = m;
         }
@@ -190,6 +205,30 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_kernel(const uint2* __restr
         const unsigned cnt = min(static_cast<unsigned>(kBatch), range.y - base);
         const unsigned live = __ballot_sync(0xFFFFFFFFu, T.x + T.y > 0.f);
         if (!live) continue;  // the warp is finished
+        const auto step = [&](unsigned id) {
+            const float4 a = s_r0[id];
+            const float4 k = s_r1[id];
+            const float bb = s_b[id];
+            float2 dx;
+            const float2 pp = splat_exponents2(a, k, make_float2(px0, px0 + 1.0f), __fsub_rn(py, a.y), dx);
+            blend_px2<kTrain>(pp, k.y, k.z, k.w, bb, T, cr, cg, cb, tf, last0, last1, base + id + 1);
+        };
+        if (kSparse && cnt <= 32) {
+            // A short round: each quarter takes its splats from its ballot, without lists.
+            const unsigned m = static_cast<unsigned>(lane) < cnt ? s_mask[lane] >> cell0 : 0u;
+            unsigned todo = 0, steps = 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const unsigned bits = __ballot_sync(0xFFFFFFFFu, (m >> ((q & 1) + (q >> 1) * kCells)) & 1u);
+                if (quarter == q) todo = bits;
+                steps = max(steps, static_cast<unsigned>(__popc(bits)));
+            }
+            for (; steps > 0; --steps) {
+                step(todo ? __ffs(todo) - 1u : static_cast<unsigned>(kBatch));
+                todo &= todo - 1;
+            }
+            continue;
+        }
         // Each quarter's splats of the round in list order, compacted once (a ballot per quarter and 32
         // staged); a finished quarter takes none. Then every list is padded with the splat that no
         // pixel takes to the longest one's length, a multiple of four.
@@ -215,14 +254,7 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_kernel(const uint2* __restr
             const unsigned id[4] = {four.x, four.y, four.z, four.w};
             // Four splats per vote on whether the warp is finished.
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float4 a = s_r0[id[u]];
-                const float4 k = s_r1[id[u]];
-                const float bb = s_b[id[u]];
-                float2 dx;
-                const float2 pp = splat_exponents2(a, k, make_float2(px0, px0 + 1.0f), __fsub_rn(py, a.y), dx);
-                blend_px2<kTrain>(pp, k.y, k.z, k.w, bb, T, cr, cg, cb, tf, last0, last1, base + id[u] + 1);
-            }
+            for (int u = 0; u < 4; ++u) step(id[u]);
             if (!__any_sync(0xFFFFFFFFu, T.x + T.y > 0.f)) break;
         }
     }
@@ -241,15 +273,11 @@ __global__ void __launch_bounds__(TW * TH / 2) blend_kernel(const uint2* __restr
     }
 }
 
-template <int TW, int TH, int kBatch>
+template <int TW, int TH, int kBatch, bool kSparse>
 void launch_shape(unsigned tiles, const uint2* ranges, const unsigned* vals, const SplatRecord* rec, const Ctrl* ctrl,
                   const ViewInfo* views, const BatchTables& tables, bool train, cudaStream_t stream) {
-    if (train)
-        launch_chained(blend_kernel<TW, TH, kBatch, true>, dim3(tiles), dim3(TW * TH / 2), stream, ranges, vals, rec,
-                       ctrl, views, tables);
-    else
-        launch_chained(blend_kernel<TW, TH, kBatch, false>, dim3(tiles), dim3(TW * TH / 2), stream, ranges, vals, rec,
-                       ctrl, views, tables);
+    const auto kernel = train ? blend_kernel<TW, TH, kBatch, true, kSparse> : blend_kernel<TW, TH, kBatch, false, kSparse>;
+    launch_chained(kernel, dim3(tiles), dim3(TW * TH / 2), stream, ranges, vals, rec, ctrl, views, tables);
 }
 
 }  // namespace
@@ -260,19 +288,17 @@ bool blend_shape_supported(int tile_w, int tile_h) {
 
 void launch_blend(unsigned tiles, const uint2* ranges, const unsigned* sorted_vals, const SplatRecord* rec,
                   const Ctrl* ctrl, const ViewInfo* views, const BatchTables& tables, int tile_w, int tile_h,
-                  int batch, bool train, cudaStream_t stream) {
+                  int batch, bool sparse, bool train, cudaStream_t stream) {
     if (tiles == 0) return;
     const bool big = batch >= 256;
-    if (tile_w == 8) {
-        if (big) launch_shape<8, 8, 256>(tiles, ranges, sorted_vals, rec, ctrl, views, tables, train, stream);
-        else launch_shape<8, 8, 128>(tiles, ranges, sorted_vals, rec, ctrl, views, tables, train, stream);
-    } else if (tile_h == 32) {
-        if (big) launch_shape<16, 32, 256>(tiles, ranges, sorted_vals, rec, ctrl, views, tables, train, stream);
-        else launch_shape<16, 32, 256>(tiles, ranges, sorted_vals, rec, ctrl, views, tables, train, stream);
-    } else {
-        if (big) launch_shape<16, 16, 256>(tiles, ranges, sorted_vals, rec, ctrl, views, tables, train, stream);
-        else launch_shape<16, 16, 128>(tiles, ranges, sorted_vals, rec, ctrl, views, tables, train, stream);
-    }
+    const auto launch = tile_w == 8    ? (sparse ? launch_shape<8, 8, 128, true>
+                                          : big  ? launch_shape<8, 8, 256, false>
+                                                 : launch_shape<8, 8, 128, false>)
+                        : tile_h == 32 ? (sparse ? launch_shape<16, 32, 256, true> : launch_shape<16, 32, 256, false>)
+                                       : (sparse ? launch_shape<16, 16, 128, true>
+                                          : big  ? launch_shape<16, 16, 256, false>
+                                                 : launch_shape<16, 16, 128, false>);
+    launch(tiles, ranges, sorted_vals, rec, ctrl, views, tables, train, stream);
 }
 
 }  // namespace ab2

@@ -771,7 +771,8 @@ int enqueue_plan(Arena& A, Slot& slot, const Plan<Src>& P, cudaStream_t st, cuda
     if (ev) AB_CUDA(cudaEventRecord(ev[2], st));
     if (!stop_after_sort)
         launch_blend(static_cast<unsigned>(P.tiles), A.ranges.p, A.pair_val[fin].p, A.rec.p, A.ctrl.p, views, tables,
-                     P.shape.tile_w, P.shape.tile_h, P.shape.blend_batch, train, st);
+                     P.shape.tile_w, P.shape.tile_h, P.shape.blend_batch, sparse_frame(P.entries, P.tiles), train,
+                     st);
     if (ev) AB_CUDA(cudaEventRecord(ev[3], st));
     AB_CUDA(cudaGetLastError());
     if (mark_slot) AB_TRY(slot.mark(st));
@@ -2008,7 +2009,8 @@ int train_backward(aniso_b200_trainer* t, const float* const* grad_images, const
         in.offs = A.offs.p;
         in.rect = rect;
         AB_CUDA(cudaMemsetAsync(t->vis_counts.p, 0, P.views.size() * sizeof(unsigned), cs));
-        launch_blend_backward(in, static_cast<unsigned>(P.tiles), P.shape.tile_w, P.shape.tile_h, t->grad_pair.p, cs);
+        launch_blend_backward(in, static_cast<unsigned>(P.tiles), P.shape.tile_w, P.shape.tile_h,
+                              sparse_frame(P.entries, P.tiles), t->grad_pair.p, cs);
         for (size_t k = 0; k < P.views.size(); ++k) {
             const unsigned s = P.views[k].scene;
             const GaussBackwardArgs ga{scenes, s, views, static_cast<unsigned>(k), slot.grads_dev(P),

@@ -373,8 +373,8 @@ __device__ __forceinline__ float sqrt_mufu(float x) {  // MUFU square root, rela
 // the bounds (in log2 units: far above the rounding of this test and of the blend's evaluation, also
 // for needles, whose terms cancel), and the extent is widened by 1e-3 of the half-width plus 0.01
 // pixel (MUFU square roots and reciprocals, relative error ~2^-22). A degenerate form (a coefficient
-// that is 0 or not finite, or not concave) keeps every cell of the bounds.
-template <int TW, int TH, int CW, int CH>
+// that is 0 or not finite, or not concave) keeps every cell of the bounds. kEllipse false: the bounds alone.
+template <int TW, int TH, int CW, int CH, bool kEllipse = true>
 __device__ __forceinline__ unsigned staged_cell_mask(const SplatRecord& r, int ox, int oy) {
     constexpr float kCut = -7.99435343685885793f;  // log2(1/255)
     constexpr int kC = TW / CW, kR = TH / CH;
@@ -389,6 +389,7 @@ __device__ __forceinline__ unsigned staged_cell_mask(const SplatRecord& r, int o
     for (int rr = 0; rr < kR; ++rr)
         if (ylo <= oy + CH * rr + CH - 1 && yhi >= oy + CH * rr) m |= cols << (kC * rr);
 
+    if (!kEllipse) return m;
     const float u = r.r0.x, v = r.r0.y, A = r.r0.z, B = r.r0.w, C = r.r1.x, L = r.r1.y;
     const float det4 = 4.f * A * C - B * B;
     if (!(A < 0.f && C < 0.f && det4 > 0.f && isfinite(A + B + C + L + det4))) return m;

@@ -190,12 +190,16 @@ size_t tile_sum_words(uint64_t tiles);
 size_t tile_chunk_entries(uint64_t capacity);
 void launch_tile_sort(const TileSortArgs& args, cudaStream_t stream);
 
+// Whether a frame has few entries (visible or not) for its tiles, so that most lists are short or empty.
+inline bool sparse_frame(uint64_t entries, uint64_t tiles) { return entries / 32 < tiles; }
+
 // Blends every tile of a batch (blockIdx = global tile); outputs go to each view's ViewInfo.
+// batch: splats staged per round; sparse (sparse_frame): the lists are short, the smaller rounds are taken.
 // train: also the float colour, final transmittance and last contributor per pixel.
 bool blend_shape_supported(int tile_w, int tile_h);
 void launch_blend(unsigned tiles, const uint2* ranges, const unsigned* sorted_vals, const SplatRecord* rec,
                   const Ctrl* ctrl, const ViewInfo* views, const BatchTables& tables, int tile_w, int tile_h,
-                  int batch, bool train, cudaStream_t stream);
+                  int batch, bool sparse, bool train, cudaStream_t stream);
 
 // ---- the adjoint ----------------------------------------------------------------------------
 struct BackwardIn {
@@ -224,7 +228,7 @@ struct RawGrads {
     unsigned pad;
 };
 // grad_pair: 9 floats per pair, at the pair's depth-ordered slot.
-void launch_blend_backward(const BackwardIn& in, unsigned tiles, int tile_w, int tile_h, float* grad_pair,
+void launch_blend_backward(const BackwardIn& in, unsigned tiles, int tile_w, int tile_h, bool sparse, float* grad_pair,
                            cudaStream_t stream);
 // One view of one scene, everything the kernel reads about them in the frame's device tables: the
 // scene's raw tensors (scenes[scene].src), the view's camera and entry base (views[view]), the

@@ -413,7 +413,6 @@ __device__ __forceinline__ void sort_chunk(const unsigned long long* src, unsign
 // One warp's sort of n (0..kShortList) pairs at src into entries at out, two pairs per lane: a pair's place
 // is the number of smaller ones, counted as the warp passes every pair round.
 constexpr unsigned kShortList = 64;
-constexpr unsigned kSparseEntries = 32;  // entries (visible or not) per tile below which a frame is sparse
 __device__ __forceinline__ void sort_short(const unsigned long long* src, unsigned n, unsigned* out) {
     const unsigned lane = threadIdx.x & 31;
     const unsigned long long x0 = lane < n ? src[lane] : kNoPair, x1 = lane + 32 < n ? src[lane + 32] : kNoPair;
@@ -609,7 +608,7 @@ void launch_tile_sort(const TileSortArgs& a, cudaStream_t stream) {
     launch_chained(scatter, dim3(std::max(1u, std::min(rounds, 148u * 32u))), dim3(kThreads), stream,
                    a.depth_key, a.rect16, a.entries, a.tables, a.cursor, a.pairs, a.offs, a.ctrl);
     const unsigned further = std::min(a.chunk_cap, 296u);
-    const bool sparse = a.entries / kSparseEntries < a.tiles;
+    const bool sparse = sparse_frame(a.entries, a.tiles);
     const unsigned list_ctas = sparse ? (a.tiles + kWarps - 1) / kWarps : a.tiles;
     launch_chained(sparse ? tile_sort_kernel<true> : tile_sort_kernel<false>, dim3(list_ctas + further), dim3(kThreads),
                    stream, a.ranges, a.tiles, a.chunks, a.chunk_cap, a.pairs, a.vals, a.ctrl);
