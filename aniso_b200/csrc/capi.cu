@@ -98,6 +98,13 @@ constexpr uint64_t kMaxPairs = 0x3FFFFFFFull;    // pair positions and the span 
 // 31 us.
 constexpr uint64_t kTileSortEntries = 8192;
 constexpr uint64_t kTileSortTiles = 1ull << 24;
+// Nor does it take frames of many entries per tile (thumbnails of large scenes): their adds crowd on few
+// counters, one after another, and their lists need merging. With the chain and with the tile sort, by
+// entries per tile: 304 and 256 us a frame at 4313 (2.2M, 480x270), 224 and 249 at 5138 (740k, 256x144), 237 and
+// 397 at 12333 (740k, 160x90), 311 and 699 at 36666 (2.2M, 160x90). The training path gains from the cut
+// rectangles in the adjoint too: forward and backward 791 and 761 us at 6666 (400k, 160x90), 863 and 922
+// at 12333 (740k, 160x90).
+constexpr uint64_t kCrowdedEntries = 4500, kCrowdedTrainEntries = 9000;
 
 // Work buffers of one frame at a time, sized for `n` entries and a pair capacity. Each sort's own
 // buffers are made when a frame first takes it (prepare).
@@ -164,8 +171,9 @@ struct Arena {
     }
 
     // Whether the tile sort takes a frame (its counters take 64 bytes a tile).
-    bool tile_sorted(uint64_t entries, uint64_t tiles) const {
-        return !ctas && entries >= kTileSortEntries && tiles <= kTileSortTiles;
+    bool tile_sorted(uint64_t entries, uint64_t tiles, bool train) const {
+        return !ctas && entries >= kTileSortEntries && tiles <= kTileSortTiles &&
+               entries <= (train ? kCrowdedTrainEntries : kCrowdedEntries) * tiles;
     }
 
     // Everything a frame of `entries` entries and `tiles` tiles needs beyond init (no list of a tile
@@ -173,7 +181,7 @@ struct Arena {
     int prepare(uint64_t entries, uint64_t tiles, uint64_t longest, bool train) {
         AB_TRY(grow(ranges, static_cast<size_t>(tiles)));
         AB_TRY(grow(pair_val[0], pair_cap));
-        if (tile_sorted(entries, tiles)) {
+        if (tile_sorted(entries, tiles, train)) {
             AB_TRY(grow(pairs, pair_cap));
             if (train) AB_TRY(grow(whole, static_cast<size_t>(std::max<int64_t>(n, 1))));
             if (longest > static_cast<uint64_t>(kTileGroup) * kTileChunk) AB_TRY(grow(merged, pair_cap));
@@ -747,7 +755,7 @@ int enqueue_plan(Arena& A, Slot& slot, const Plan<Src>& P, cudaStream_t st, cuda
     BatchTables tables;
     AB_TRY(A.prepare(P.entries, P.tiles, P.longest(), train));
     const unsigned entries = static_cast<unsigned>(P.entries), tiles = static_cast<unsigned>(P.tiles);
-    const bool by_tile = A.tile_sorted(P.entries, P.tiles);
+    const bool by_tile = A.tile_sorted(P.entries, P.tiles, train);
     unsigned zero_words = 0;
     const PassCounts first = by_tile ? PassCounts{} : first_pass_counts(A, entries, P.short_depth, &zero_words);
     // A frame that is only sorted shows its pairs, so it keeps the whole rectangles.
@@ -1991,7 +1999,7 @@ int train_backward(aniso_b200_trainer* t, const float* const* grad_images, const
         fresh[k] = grads[s].fresh != 0 && k == P.scenes[s].view_begin;
     }
     // Where the forward's sort left the entries' gradient slots (BackwardIn).
-    const bool by_tile = A.tile_sorted(P.entries, P.tiles);
+    const bool by_tile = A.tile_sorted(P.entries, P.tiles, true);
     const unsigned* rank = by_tile ? nullptr : A.rank.p;
     const unsigned long long* rect = by_tile ? A.rect16.p : A.rect_sorted.p;
     const unsigned long long* whole = by_tile ? A.whole.p : nullptr;
