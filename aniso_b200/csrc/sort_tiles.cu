@@ -111,8 +111,11 @@ __global__ void __launch_bounds__(kScanThreads) tile_scan_kernel(const unsigned*
 
 // ---- scatter -------------------------------------------------------------------------------------
 
-constexpr unsigned kScatterEntries = kThreads;  // entries per CTA and round
+constexpr unsigned kScatterLanes = 32, kScatterFewLanes = 8;  // entries per warp and round, and in a small frame
 constexpr unsigned kFewEntries = 1u << 21;  // up to here a warp keeps four pairs per lane in flight, above it two
+// Up to here a warp takes 8 entries at a time, above it 32: with 32 a frame of so few entries does not give
+// every SM a CTA (20k splats of 800 tiles each, 1920x1080: 240 us of scatter; the frame 611 -> 480 us).
+constexpr unsigned kFewestEntries = 148 * kThreads;
 constexpr unsigned kLargeArea = 1024;  // an entry of more tiles is left to the whole CTA
 
 // Tile k of a rectangle w tiles wide with corner tile org, in a view of tx tiles per row.
@@ -132,7 +135,7 @@ __device__ __forceinline__ unsigned tile_of(unsigned k, unsigned org, unsigned w
 // (Spreading the pairs of a CTA's 256 to 1024 entries over its threads takes a fifth of the instructions
 // and is no faster; nor is ranking small entries' pairs as they are counted, which saves the scatter
 // four fifths of its adds: the scattered accesses themselves bound it.)
-template <int kScatterPairs>
+template <int kScatterPairs, unsigned kLanes>
 __global__ void __launch_bounds__(kThreads) tile_scatter_kernel(const unsigned* __restrict__ depth_key,
                                                                 const unsigned long long* __restrict__ rect16,
                                                                 unsigned entries, BatchTables tables,
@@ -142,15 +145,16 @@ __global__ void __launch_bounds__(kThreads) tile_scatter_kernel(const unsigned* 
     chain_entry();
     __shared__ unsigned s_total[kWarps];
     __shared__ unsigned s_base;
+    constexpr unsigned kScatterEntries = kLanes * kWarps;  // per CTA and round
     __shared__ unsigned s_large[kScatterEntries];
     __shared__ unsigned s_large_count;
     if (ctrl->flags & kFlagOverflow) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned rounds = entries / kScatterEntries + (entries % kScatterEntries != 0);
     for (unsigned round = blockIdx.x; round < rounds; round += gridDim.x) {
-        const unsigned first = round * kScatterEntries + warp * 32, e = first + lane;
+        const unsigned first = round * kScatterEntries + warp * kLanes, e = first + lane;
         if (tid == 0) s_large_count = 0;
-        const unsigned key = e < entries ? depth_key[e] : kCulledKey;
+        const unsigned key = lane < kLanes && e < entries ? depth_key[e] : kCulledKey;
         const bool visible = key != kCulledKey;
         unsigned org = 0, width = 1, tx = 0, area = 0;
         if (visible) {
@@ -184,7 +188,7 @@ __global__ void __launch_bounds__(kThreads) tile_scatter_kernel(const unsigned* 
         }
         {
             const bool large = area > kLargeArea;
-            if (large) s_large[atomicAdd(&s_large_count, 1u)] = static_cast<unsigned>(warp * 32 + lane);
+            if (large) s_large[atomicAdd(&s_large_count, 1u)] = static_cast<unsigned>(warp * kLanes + lane);
             const unsigned spread = large ? 0u : area;
             const unsigned incl = warp_incl_scan(spread);
             const unsigned excl = incl - spread, total = __shfl_sync(0xFFFFFFFFu, incl, 31);
@@ -470,10 +474,9 @@ __global__ void __launch_bounds__(kThreads, 8) tile_sort_kernel(const uint2* __r
             return;
         }
         const unsigned first = blockIdx.x * kTiles, end = min(first + kTiles, tiles), mine = first + (threadIdx.x >> 5);
-        if (mine < end) {
-            const uint2 r = ranges[mine];
-            if (r.y - r.x <= kShortList) sort_short(pairs + r.x, r.y - r.x, vals + r.x);
-        }
+        const uint2 own = mine < end ? ranges[mine] : make_uint2(0u, 0u);
+        if (own.y - own.x <= kShortList) sort_short(pairs + own.x, own.y - own.x, vals + own.x);
+        if (!__syncthreads_or(own.y - own.x > kShortList)) return;
         for (unsigned t = first; t < end; ++t) {
             const uint2 r = ranges[t];
             const unsigned n = r.y - r.x;
@@ -494,28 +497,23 @@ __global__ void __launch_bounds__(kThreads, 8) tile_sort_kernel(const uint2* __r
     }
 }
 
-// Items of the m sorted pairs at s (padded places) that are smaller than x.
-__device__ __forceinline__ unsigned lower_count(const unsigned long long* s, unsigned m, unsigned long long x) {
-    unsigned lo = 0, hi = m;
-    while (lo < hi) {
-        const unsigned mid = (lo + hi) >> 1;
-        if (s[padded(mid)] < x) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
 // Merges the sorted chunks of every list of several: the place of a pair is its place in its own
-// chunk plus, for every other chunk of its group (kTileGroup chunks), the number of smaller pairs there
-// (a search in a copy of that chunk in shared memory). A list of one group is written as sorted entries;
-// a group of a longer one as pairs to `merged`, for tile_merge_groups_kernel.
+// chunk plus, for every other chunk of its group (kTileGroup chunks), the number of smaller pairs there.
+// Both chunks lie in shared memory and the CTA merges them, sixteen outputs per thread from a merge-path
+// search: each pair of its own is passed once and gets the other chunk's place of the moment. A list of one
+// group is written as sorted entries; a group of a longer one as pairs to `merged`, for
+// tile_merge_groups_kernel. (With a search of eleven steps for every pair instead, 740k splats
+// within 70 pixels take 1026 us a frame, with the merges 914; within 140 pixels 462 and 444; 64 views of 1M
+// 5.91 and 5.86 ms.)
 __global__ void __launch_bounds__(kThreads) tile_merge_kernel(const uint2* __restrict__ ranges,
                                                               const uint2* __restrict__ chunks, unsigned chunk_cap,
                                                               const unsigned long long* __restrict__ pairs,
                                                               unsigned long long* __restrict__ merged,
                                                               unsigned* __restrict__ vals, const Ctrl* ctrl) {
     chain_entry();
-    __shared__ unsigned long long s_pair[kTileChunk + kTileChunk / 8];
+    constexpr unsigned kOutputs = 2 * kItems;  // of two whole chunks, per thread
+    __shared__ unsigned long long s_own[kTileChunk + kTileChunk / 8], s_other[kTileChunk + kTileChunk / 8];
+    __shared__ unsigned s_place[kTileChunk];
     if (ctrl->flags & kFlagOverflow) return;
     const unsigned count = min(ctrl->chunk_count, chunk_cap);
     for (unsigned c = blockIdx.x; c < count; c += gridDim.x) {
@@ -524,30 +522,45 @@ __global__ void __launch_bounds__(kThreads) tile_merge_kernel(const uint2* __res
         const unsigned of = (r.y - r.x + kTileChunk - 1) / kTileChunk;  // chunks of the list
         const unsigned g0 = ch.y / kTileGroup * kTileGroup, g1 = min(of, g0 + kTileGroup);
         const unsigned at = r.x + ch.y * kTileChunk, m = min(kTileChunk, r.y - at);
-        unsigned long long x[kItems];
-        unsigned place[kItems];
-#pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            const unsigned i = k * kThreads + threadIdx.x;
-            x[k] = i < m ? pairs[at + i] : 0ull;
-            place[k] = i;
+        __syncthreads();
+        for (unsigned i = threadIdx.x; i < m; i += kThreads) {
+            s_own[padded(i)] = pairs[at + i];
+            s_place[i] = i;
         }
         for (unsigned o = g0; o < g1; ++o) {
             if (o == ch.y) continue;
             const unsigned oat = r.x + o * kTileChunk, om = min(kTileChunk, r.y - oat);
             __syncthreads();
-            for (unsigned i = threadIdx.x; i < om; i += kThreads) s_pair[padded(i)] = pairs[oat + i];
+            for (unsigned i = threadIdx.x; i < om; i += kThreads) s_other[padded(i)] = pairs[oat + i];
             __syncthreads();
+            const unsigned diag = threadIdx.x * kOutputs;
+            if (diag >= m + om) continue;
+            unsigned lo = diag > om ? diag - om : 0u, hi = min(diag, m);
+            while (lo < hi) {  // own pairs among the first diag outputs
+                const unsigned mid = (lo + hi) >> 1;
+                if (s_own[padded(mid)] < s_other[padded(diag - 1 - mid)]) lo = mid + 1;
+                else hi = mid;
+            }
+            unsigned a = lo, b = diag - lo;
+            unsigned long long va = a < m ? s_own[padded(a)] : kNoPair, vb = b < om ? s_other[padded(b)] : kNoPair;
 #pragma unroll
-            for (int k = 0; k < kItems; ++k)
-                if (k * kThreads + threadIdx.x < m) place[k] += lower_count(s_pair, om, x[k]);
+            for (unsigned k = 0; k < kOutputs; ++k) {
+                const bool own = va < vb;
+                if (own) s_place[a] += b;
+                a += own;
+                b += !own;
+                const unsigned p = own ? a : b, end = own ? m : om;
+                const unsigned long long next = p < end ? (own ? s_own : s_other)[padded(p)] : kNoPair;
+                va = own ? next : va;
+                vb = own ? vb : next;
+            }
         }
+        __syncthreads();
         const unsigned out = r.x + g0 * kTileChunk;
-#pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            if (k * kThreads + threadIdx.x >= m) continue;
-            if (of <= kTileGroup) vals[out + place[k]] = static_cast<unsigned>(x[k]);
-            else merged[out + place[k]] = x[k];
+        for (unsigned i = threadIdx.x; i < m; i += kThreads) {
+            const unsigned long long x = s_own[padded(i)];
+            if (of <= kTileGroup) vals[out + s_place[i]] = static_cast<unsigned>(x);
+            else merged[out + s_place[i]] = x;
         }
     }
 }
@@ -603,18 +616,24 @@ void launch_tile_sort(const TileSortArgs& a, cudaStream_t stream) {
     launch_chained(tile_scan_kernel, dim3(ctas), dim3(kScanThreads), stream, a.counts, a.tiles,
                    sums ? static_cast<const unsigned*>(a.sums) : nullptr, a.ranges, a.cursor, a.chunks, a.chunk_cap,
                    a.capacity, a.ctrl);
-    const unsigned rounds = static_cast<unsigned>((static_cast<uint64_t>(a.entries) + kScatterEntries - 1) / kScatterEntries);
-    const auto scatter = a.entries <= kFewEntries ? tile_scatter_kernel<4> : tile_scatter_kernel<2>;
+    const bool few = a.entries <= kFewestEntries;
+    const uint64_t per = (few ? kScatterFewLanes : kScatterLanes) * kWarps;
+    const unsigned rounds = static_cast<unsigned>((a.entries + per - 1) / per);
+    const auto scatter = few                        ? tile_scatter_kernel<4, kScatterFewLanes>
+                         : a.entries <= kFewEntries ? tile_scatter_kernel<4, kScatterLanes>
+                                                    : tile_scatter_kernel<2, kScatterLanes>;
     launch_chained(scatter, dim3(std::max(1u, std::min(rounds, 148u * 32u))), dim3(kThreads), stream,
                    a.depth_key, a.rect16, a.entries, a.tables, a.cursor, a.pairs, a.offs, a.ctrl);
-    const unsigned further = std::min(a.chunk_cap, 296u);
+    // In step with the capacity, which grows with the pairs: 296 CTAs for every frame left 300k splats of 59 tiles
+    // each waiting for their further chunks (556 us a frame, with these two grids 504).
+    const unsigned further = std::max(1u, std::min(a.chunk_cap / 8, 148u * 8u));
     const bool sparse = sparse_frame(a.entries, a.tiles);
     const unsigned list_ctas = sparse ? (a.tiles + kWarps - 1) / kWarps : a.tiles;
     launch_chained(sparse ? tile_sort_kernel<true> : tile_sort_kernel<false>, dim3(list_ctas + further), dim3(kThreads),
                    stream, a.ranges, a.tiles, a.chunks, a.chunk_cap, a.pairs, a.vals, a.ctrl);
     if (a.longest <= kTileChunk) return;
-    launch_chained(tile_merge_kernel, dim3(std::min(a.chunk_cap, 592u)), dim3(kThreads), stream, a.ranges, a.chunks,
-                   a.chunk_cap, a.pairs, a.merged, a.vals, a.ctrl);
+    launch_chained(tile_merge_kernel, dim3(std::max(1u, std::min(a.chunk_cap / 2, 148u * 5u))), dim3(kThreads), stream,
+                   a.ranges, a.chunks, a.chunk_cap, a.pairs, a.merged, a.vals, a.ctrl);
     if (a.longest <= kTileGroup * kTileChunk) return;
     launch_chained(tile_merge_groups_kernel, dim3(std::min(a.chunk_cap, 592u)), dim3(kThreads), stream, a.ranges,
                    a.chunks, a.chunk_cap, a.merged, a.vals, a.ctrl);
