@@ -98,13 +98,15 @@ constexpr uint64_t kMaxPairs = 0x3FFFFFFFull;    // pair positions and the span 
 // 31 us.
 constexpr uint64_t kTileSortEntries = 8192;
 constexpr uint64_t kTileSortTiles = 1ull << 24;
-// Nor does it take frames of many entries per tile (thumbnails of large scenes): their adds crowd on few
-// counters, one after another, and their lists need merging. With the chain and with the tile sort, by
-// entries per tile: 304 and 256 us a frame at 4313 (2.2M, 480x270), 224 and 249 at 5138 (740k, 256x144), 237 and
-// 397 at 12333 (740k, 160x90), 311 and 699 at 36666 (2.2M, 160x90). The training path gains from the cut
-// rectangles in the adjoint too: forward and backward 791 and 761 us at 6666 (400k, 160x90), 863 and 922
-// at 12333 (740k, 160x90).
-constexpr uint64_t kCrowdedEntries = 4500, kCrowdedTrainEntries = 9000;
+// Nor does it take frames of many visible entries per tile (Plan::crowd): thumbnails, and large scenes seen from
+// afar. Their adds crowd on few counters, one after another, and their lists need merging. With the chain
+// and with the tile sort, views from within scenes whose boxes leave kVisible of the entries visible, by
+// visible entries per tile: 304 and 256 us a frame at 1940 (2.2M, 480x270), 224 and 249 at 2310 (740k, 256x144),
+// 237 and 397 at 5550 (740k, 160x90), 311 and 699 at 16500 (2.2M, 160x90). The training path gains from the cut
+// rectangles in the adjoint too: forward and backward 791 and 761 us at 3000 (400k, 160x90), 863 and 922
+// at 5550 (740k, 160x90).
+constexpr double kCrowdedEntries = 2000, kCrowdedTrainEntries = 4000;
+constexpr double kVisible = 0.45;  // of a scene's Gaussians, from within it (43% at the ring views measured)
 
 // Work buffers of one frame at a time, sized for `n` entries and a pair capacity. Each sort's own
 // buffers are made when a frame first takes it (prepare).
@@ -170,18 +172,13 @@ struct Arena {
         return 0;
     }
 
-    // Whether the tile sort takes a frame (its counters take 64 bytes a tile).
-    bool tile_sorted(uint64_t entries, uint64_t tiles, bool train) const {
-        return !ctas && entries >= kTileSortEntries && tiles <= kTileSortTiles &&
-               entries <= (train ? kCrowdedTrainEntries : kCrowdedEntries) * tiles;
-    }
-
-    // Everything a frame of `entries` entries and `tiles` tiles needs beyond init (no list of a tile
-    // longer than `longest`): nothing is allocated while the frame is enqueued or captured after this.
-    int prepare(uint64_t entries, uint64_t tiles, uint64_t longest, bool train) {
+    // Everything a frame of `tiles` tiles, sorted by the tile sort or (by_tile false) by the LSD chain, needs
+    // beyond init (no list of a tile longer than `longest`): nothing is allocated while the frame is enqueued
+    // or captured after this.
+    int prepare(bool by_tile, uint64_t tiles, uint64_t longest, bool train) {
         AB_TRY(grow(ranges, static_cast<size_t>(tiles)));
         AB_TRY(grow(pair_val[0], pair_cap));
-        if (tile_sorted(entries, tiles, train)) {
+        if (by_tile) {
             AB_TRY(grow(pairs, pair_cap));
             if (train) AB_TRY(grow(whole, static_cast<size_t>(std::max<int64_t>(n, 1))));
             if (longest > static_cast<uint64_t>(kTileGroup) * kTileChunk) AB_TRY(grow(merged, pair_cap));
@@ -346,7 +343,7 @@ void enqueue_tile_sort(Arena& A, unsigned entries, unsigned longest, unsigned ti
 // digits taking few values, so one atomic per key contends -- 0.177 ms against 0.139 ms for the
 // sort of the 740k / 1280x720 frame, when this chain sorted it.) A frame of at most bin_max_tiles() tiles (A.bins_for) takes
 // the one-pass tile binning after the expansion instead of the tile passes and the ranges.
-// short_depth: every visible key is below 2^27 (Plan::bound_depth), so three 9-bit depth passes
+// short_depth: every visible key is below 2^27 (Plan::bound_views), so three 9-bit depth passes
 // replace the four 8-bit ones (0.119 -> 0.111 ms of sort for the 740k frame, when this chain sorted it). Where the
 // persistent sort is selected (A.ctas), it replaces this whole sequence with one launch and the
 // same outputs.
@@ -492,6 +489,39 @@ bool depth_short(const PositionBox& box, const CamParams& cam) {
     return z + 1e-5 * mag + 1.0 < limit;  // false for a NaN
 }
 
+// How densely a view's n Gaussians lie on its tiles: the tiles that the scene's box covers, projected at the
+// depth of its centre, and the entries there (those beside the view left out). Every tile and kVisible of
+// the entries where the box is unknown or a corner is not in front of the camera. (An estimate: it chooses
+// how a frame is sorted, not what it shows.)
+struct Reach {
+    double entries, tiles;
+};
+Reach reach_of(const PositionBox* box, const CamParams& cam, double n, int tile_w, int tile_h) {
+    const int size[2] = {cam.tilesX, cam.tilesY}, tile[2] = {tile_w, tile_h};
+    const double f[2] = {cam.fx, cam.fy}, centre[2] = {cam.cx, cam.cy};
+    const Reach all{kVisible * n, static_cast<double>(size[0]) * size[1]};
+    if (!box || !box->finite) return all;
+    double mid[3], half[3];  // of the box along the camera's axes
+    for (int r = 0; r < 3; ++r) {
+        mid[r] = cam.t[r];
+        half[r] = 0.0;
+        for (int i = 0; i < 3; ++i) {
+            mid[r] += cam.R[3 * r + i] * 0.5 * (box->lo[i] + box->hi[i]);
+            half[r] += std::fabs(cam.R[3 * r + i]) * 0.5 * (box->hi[i] - box->lo[i]);
+        }
+    }
+    if (!(mid[2] - half[2] > 0.2)) return all;
+    Reach seen{n, 1.0};
+    for (int k = 0; k < 2; ++k) {
+        const double at = (f[k] * mid[k] / mid[2] + centre[k]) / tile[k], reach = f[k] * half[k] / mid[2] / tile[k];
+        const double inside = std::min(at + reach, static_cast<double>(size[k])) - std::max(at - reach, 0.0);
+        if (!(inside >= 0.0)) return at + reach < 0.0 || at - reach > size[k] ? Reach{0.0, 0.0} : all;
+        seen.entries *= std::min(1.0, std::max(inside, 1.0) / std::max(2.0 * reach, 1.0));
+        seen.tiles *= std::max(inside, 1.0);
+    }
+    return seen;
+}
+
 constexpr uint64_t kPrePairGaussians = 1u << 19;
 constexpr int kPrePairViews = 4;
 
@@ -504,9 +534,10 @@ struct Plan {
     std::vector<unsigned> entry_base, tile_base, tiles_x;
     std::vector<RawGrads> grads;  // the backward's gradient buffers, one per scene (empty otherwise)
     uint64_t entries = 0, tiles = 0;
+    double crowd = 0;          // visible entries per tile, about, where they lie (bound_views)
     unsigned pre_blocks = 0;
     int pre_groups = 1;        // Gaussians per thread of the preprocess
-    bool short_depth = false;  // three 9-bit depth passes (bound_depth)
+    bool short_depth = false;  // three 9-bit depth passes (bound_views)
 
     // srcs[s], stored degree deg[s]; view k of scene view_scene[k] (consecutive per scene).
     int build(const std::vector<Src>& srcs, const std::vector<int>& deg, const int32_t* view_scene, int n_views,
@@ -546,6 +577,7 @@ struct Plan {
             if (entries > kMaxEntries || tiles > kMaxEntries)
                 return fail(ANISO_B200_ERR_ARGUMENT, "more than 2^32 entries or tiles in one batch");
         }
+        crowd = kVisible * static_cast<double>(entries) / std::max(static_cast<double>(tiles), 1.0);
         // Two Gaussians per thread of the preprocess where there are enough to fill the chip all the same
         // and each has few views: 407 against 430 us per 2.2M frame, 14.95 against 15.08 ms for a training
         // batch of 3 views per scene; but 49.4 against 46.6 us per 100k frame, 2.34 against 2.29 ms for
@@ -573,11 +605,25 @@ struct Plan {
     // depths below 8192 for the view's camera, and the frame has at most kProducerCountMax entries
     // (larger frames' 9-bit passes were measured slower: the 64-view 1M batch 8.69 -> 8.75 ms when the LSD
     // chain sorted it).
-    // Without a call (the training path's positions change every step) the frame keeps 8-bit passes.
-    void bound_depth(const std::vector<const PositionBox*>& boxes) {
+    // Also estimates how crowded the frame's tiles are. Without a call (the training path's positions change
+    // every step) the frame keeps 8-bit passes and counts every tile.
+    void bound_views(const std::vector<const PositionBox*>& boxes) {
         short_depth = entries > 0 && entries <= kProducerCountMax;
-        for (const auto& v : views)
-            if (v.scene >= boxes.size() || !boxes[v.scene] || !depth_short(*boxes[v.scene], v.cam)) short_depth = false;
+        double seen = 0, reached = 0;
+        for (const auto& v : views) {
+            const PositionBox* box = v.scene < boxes.size() ? boxes[v.scene] : nullptr;
+            if (!box || !depth_short(*box, v.cam)) short_depth = false;
+            const Reach r = reach_of(box, v.cam, v.n, shape.tile_w, shape.tile_h);
+            seen += r.entries;
+            reached += r.tiles;
+        }
+        crowd = reached > 0 ? seen / reached : 0.0;
+    }
+
+    // Whether the tile sort takes the frame.
+    bool by_tile(const Arena& A, bool train) const {
+        return !A.ctas && entries >= kTileSortEntries && tiles <= kTileSortTiles &&
+               crowd <= (train ? kCrowdedTrainEntries : kCrowdedEntries);
     }
 
     // The most entries a view has: no tile's list is longer.
@@ -615,7 +661,8 @@ struct Plan {
                 return false;
         return shape.tile_w == o.shape.tile_w && shape.tile_h == o.shape.tile_h &&
                shape.blend_batch == o.shape.blend_batch && shape.radix_bits == o.shape.radix_bits &&
-               rendered_degree() == o.rendered_degree() && short_depth == o.short_depth;
+               rendered_degree() == o.rendered_degree() && short_depth == o.short_depth &&
+               (crowd > kCrowdedEntries) == (o.crowd > kCrowdedEntries);
     }
 };
 
@@ -753,9 +800,9 @@ int enqueue_plan(Arena& A, Slot& slot, const Plan<Src>& P, cudaStream_t st, cuda
     const ViewInfo* views = nullptr;
     const BatchScene<Src>* scenes = nullptr;
     BatchTables tables;
-    AB_TRY(A.prepare(P.entries, P.tiles, P.longest(), train));
+    const bool by_tile = P.by_tile(A, train);
+    AB_TRY(A.prepare(by_tile, P.tiles, P.longest(), train));
     const unsigned entries = static_cast<unsigned>(P.entries), tiles = static_cast<unsigned>(P.tiles);
-    const bool by_tile = A.tile_sorted(P.entries, P.tiles, train);
     unsigned zero_words = 0;
     const PassCounts first = by_tile ? PassCounts{} : first_pass_counts(A, entries, P.short_depth, &zero_words);
     // A frame that is only sorted shows its pairs, so it keeps the whole rectangles.
@@ -1241,7 +1288,7 @@ int single_plan(aniso_b200_scene* s, const aniso_b200_camera* camera, const anis
     if (options && options->sh_degree < 0) return fail(ANISO_B200_ERR_ARGUMENT, "sh_degree must be >= 0");
     const int32_t vs = 0;
     AB_TRY(P.build({s->view()}, {s->degree}, &vs, 1, camera, scene_shape(options)));
-    P.bound_depth({&s->box});
+    P.bound_views({&s->box});
     return 0;
 }
 
@@ -1633,7 +1680,7 @@ int aniso_b200_sort_projection(int64_t n, const uint32_t* tiles_touched, const u
     cudaStream_t st = nullptr;
     const BatchTables tables{dtab.p, dtab.p + 1, dtab.p + 2, 1u};
     const unsigned T = static_cast<unsigned>(tiles_x) * static_cast<unsigned>(tiles_y);
-    AB_TRY(A.prepare(0, T, 0, false));  // the LSD chain, whatever n
+    AB_TRY(A.prepare(false, T, 0, false));  // the LSD chain, whatever n
     launch_frame_begin(A.ctrl.p, nullptr, 0u, A.ranges.p, T, st);
     launch_projection_keys(n, dtt.p, ddepth.p, drect.p, A.depth_key.p, A.rect16.p, st,
                            short_depth ? kDepthKeyBase : 0u);
@@ -1722,7 +1769,7 @@ int aniso_b200_batch_render(aniso_b200_batch* b, const aniso_b200_camera* camera
     AB_TRY(P.build(srcs, degs, b->view_scene.data(), static_cast<int>(b->view_scene.size()), cameras, b->shape));
     std::vector<const PositionBox*> boxes;
     for (auto* s : b->scenes) boxes.push_back(&s->box);
-    P.bound_depth(boxes);
+    P.bound_views(boxes);
     for (size_t k = 0; k < P.views.size(); ++k) {
         if (!rgb_device[k]) return fail(ANISO_B200_ERR_ARGUMENT, "an output buffer is NULL");
         P.views[k].rgb8 = rgb_device[k];
@@ -1751,7 +1798,7 @@ int aniso_b200_batch_render(aniso_b200_batch* b, const aniso_b200_camera* camera
         // pinned blob at every replay, and each replay refreshes that blob first.
         // Every allocation the sequence needs happens first: none may happen while capturing.
         AB_TRY(b->graph_slot.stage(P));
-        AB_TRY(b->arena.prepare(P.entries, P.tiles, P.longest(), false));
+        AB_TRY(b->arena.prepare(P.by_tile(b->arena, false), P.tiles, P.longest(), false));
         cudaGraph_t g = nullptr;
         AB_CUDA(cudaStreamBeginCapture(b->capture_stream, cudaStreamCaptureModeThreadLocal));
         const int rc = enqueue_plan(b->arena, b->graph_slot, P, b->capture_stream, nullptr, nullptr, false, false,
@@ -1887,7 +1934,7 @@ int record_graph(aniso_b200_trainer* t, cudaGraphExec_t* exec, F&& enqueue) {
 // the launch geometry or the work buffers changed, else replayed after restaging the graph's slot.
 int train_forward_graph(aniso_b200_trainer* t, const Plan<RawParams>& P, cudaStream_t st, int* fin) {
     Arena& A = t->arena;
-    AB_TRY(A.prepare(P.entries, P.tiles, P.longest(), true));
+    AB_TRY(A.prepare(P.by_tile(A, true), P.tiles, P.longest(), true));
     AB_TRY(t->graph_slot_f.stage(P));
     if (!t->fwd_graph || t->fwd_gen != A.gen || !P.same_geometry(t->fwd_plan)) {
         if (t->fwd_graph) {
@@ -1999,7 +2046,7 @@ int train_backward(aniso_b200_trainer* t, const float* const* grad_images, const
         fresh[k] = grads[s].fresh != 0 && k == P.scenes[s].view_begin;
     }
     // Where the forward's sort left the entries' gradient slots (BackwardIn).
-    const bool by_tile = A.tile_sorted(P.entries, P.tiles, true);
+    const bool by_tile = P.by_tile(A, true);
     const unsigned* rank = by_tile ? nullptr : A.rank.p;
     const unsigned long long* rect = by_tile ? A.rect16.p : A.rect_sorted.p;
     const unsigned long long* whole = by_tile ? A.whole.p : nullptr;
