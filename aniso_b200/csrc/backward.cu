@@ -194,10 +194,6 @@ __global__ void __launch_bounds__(TW * TH / 2, TW * TH == 512 ? 3 : 0) blend_bac
         st.gg.y = vi.grad_img[3 * p + 1];
         st.gb.y = vi.grad_img[3 * p + 2];
     }
-    // An infinite or NaN gradient times a weight of zero is NaN: where the warp holds one, a lane whose
-    // pixels a splat does not apply to adds zeros to its sums all the same, in a walk of its own (496 -> 502 us
-    // of adjoint blend at 2.2M / 1280x720; with the selects in the one walk 508).
-    const bool hostile = __any_sync(0xFFFFFFFFu, !isfinite(st.gr.x + st.gg.x + st.gb.x + st.gr.y + st.gg.y + st.gb.y));
     if (tid == 0) {
         sh.maxlast = range.x;
         sh.r0[kBatch] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -357,7 +353,12 @@ __global__ void __launch_bounds__(TW * TH / 2, TW * TH == 512 ? 3 : 0) blend_bac
                 if (i < last_own) *last = ninth;
             }
         };
-        if (hostile) walk(std::true_type{});
+        // An infinite or NaN gradient times a weight of zero is NaN: where the warp holds one, a lane whose
+        // pixels a splat does not apply to adds zeros to its sums all the same, in a walk of its own. (Asked for
+        // only here, so that the gradients' loads stay in flight over the staging: asked for before it, 502
+        // instead of 495 us of adjoint blend at 2.2M / 1280x720; selects in the one walk 506.)
+        const float grads = st.gr.x + st.gg.x + st.gb.x + st.gr.y + st.gg.y + st.gb.y;
+        if (__any_sync(0xFFFFFFFFu, !isfinite(grads))) walk(std::true_type{});
         else walk(std::false_type{});
         __syncthreads();
         // Fixed-order sum over the quarters and warps; every pair of the round is written. Neighbouring
