@@ -624,9 +624,9 @@ void launch_tile_sort(const TileSortArgs& a, cudaStream_t stream) {
                                                     : tile_scatter_kernel<2, kScatterLanes>;
     launch_chained(scatter, dim3(std::max(1u, std::min(rounds, 148u * 32u))), dim3(kThreads), stream,
                    a.depth_key, a.rect16, a.entries, a.tables, a.cursor, a.pairs, a.offs, a.ctrl);
-    // In step with the capacity, which grows with the pairs: 296 CTAs for every frame left 300k splats of 59 tiles
-    // each waiting for their further chunks (556 us a frame, with these two grids 504).
-    const unsigned further = std::max(1u, std::min(a.chunk_cap / 8, 148u * 8u));
+    // More in step with the capacity, which grows with the pairs: 296 CTAs left 300k splats of 59 tiles each
+    // waiting for their further chunks (556 us a frame, with this and the merge's grid 504).
+    const unsigned further = std::min(a.chunk_cap, std::max(296u, std::min(a.chunk_cap / 8, 148u * 8u)));
     const bool sparse = sparse_frame(a.entries, a.tiles);
     const unsigned list_ctas = sparse ? (a.tiles + kWarps - 1) / kWarps : a.tiles;
     launch_chained(sparse ? tile_sort_kernel<true> : tile_sort_kernel<false>, dim3(list_ctas + further), dim3(kThreads),
