@@ -259,8 +259,9 @@ __device__ __forceinline__ unsigned axis_bounds(float centre, float cov, float t
 constexpr int kMaxStagedViews = 64;  // cameras of a scene's views kept in shared memory
 constexpr int kPreThreads = 128;
 constexpr int kPreWarps = kPreThreads / 32;
-constexpr int kPreSlotBits = 10;  // of a queue item: the Gaussian's place in the CTA; the view above it
+constexpr int kPreSlotBits = 8;  // of a queue item: the Gaussian's place in the CTA; the view of its scene above it
 static_assert(2 * kPreThreads <= 1 << kPreSlotBits, "a place fits its bits");
+static_assert(32 - kPreSlotBits >= 24, "a scene may have 2^24 views in a batch");
 
 // The projection of one entry that passed the early test, by any lane of the warp (the Gaussian's
 // activated position / opacity and covariance come from its owner lane through shared memory):
