@@ -7,8 +7,8 @@ Each csrc/*.cu file is compiled separately (in parallel) with -O3, IEEE division
 (no --use_fast_math: the projection must round like the reference kernel built without it),
 -lineinfo for ncu source correlation, and -Xptxas -v, whose register / spill / shared-memory
 report is written to _build/ptxas.txt. csrc/peaks/peaks.cu becomes libaniso_b200_peaks.so, the
-ex2 / FMA throughput probe whose rates are the blend's compute-roofline denominators (the
-renderer does not link it). The GpuRenderer shim (shim/gpu_render_shim.cpp) is built
+ex2 / FMA throughput probe whose rates the bench reports beside the blend's issue rate (the renderer
+does not link it). The GpuRenderer shim (shim/gpu_render_shim.cpp) is built
 by oracle/Makefile's `dropin` target, against the reference's headers.
 """
 from __future__ import annotations

@@ -3,9 +3,9 @@
 // Everything renders through one plan: V views of S scenes. A frame is a fixed, host-sync-free
 // sequence of kernels on one stream (capturable in a CUDA graph), launched with programmatic
 // stream serialisation: the frame's start (upload of the plan's view table, clears of the control block
-// and the counts), preprocess, the sort (tile ranges, pair scatter, per-tile sort and merge; in small
-// frames the LSD chain: depth passes, pair scan, pair expansion, tile passes or binning), blend. After a synchronous frame one more kernel hands the control block
-// to the host. Data-dependent sizes (visible entries, pairs) stay on the
+// and the counts), preprocess, the sort (tile ranges, pair scatter, per-tile sort and merge; in small and
+// in crowded frames the LSD chain: depth passes, pair scan, pair expansion, tile passes or binning), blend.
+// After a synchronous frame one more kernel hands the control block to the host. Data-dependent sizes (visible entries, pairs) stay on the
 // device; grids are sized for capacity and surplus blocks exit at once. The reference instead reads
 // the pair count back mid-frame (gpu_render.cu:329) to size its buffers; here a frame whose pairs
 // exceed the capacity sets an overflow flag instead of writing them, and the host grows the

@@ -41,7 +41,7 @@ struct CamParams {
 };
 
 struct SceneView {
-    static constexpr bool kCrossXz = true;  // rounding of the covariance (covariance() of the preprocess)
+    static constexpr bool kCrossXz = true;  // rounding of the covariance, not RawParams' (covariance() of the preprocess)
     const float4* pos_op;
     const float4* scale;
     const float4* rot;

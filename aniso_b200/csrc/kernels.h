@@ -179,7 +179,7 @@ struct TileSortArgs {
     uint2* chunks;                     // [chunk_cap]: tile_chunk_entries(capacity)
     unsigned chunk_cap;
     unsigned long long* pairs;         // [capacity]
-    unsigned long long* merged;        // [capacity] if longest > tile_group_pairs(), else NULL
+    unsigned long long* merged;        // [capacity] if longest > kTileGroup * kTileChunk, else NULL
     unsigned* vals;                    // [capacity]
     unsigned* offs;                    // [entries] or NULL
     unsigned capacity;
@@ -227,7 +227,8 @@ struct RawGrads {
     unsigned fresh;  // 1: the buffers hold zeros (the scene's first view of a fresh gradient): store, do not read
     unsigned pad;
 };
-// grad_pair: 9 floats per pair, at the pair's depth-ordered slot.
+// grad_pair: 9 floats per pair, at the pair's slot (BackwardIn): an entry's are contiguous, the entries' in depth
+// order with the LSD chain, in any order with the tile sort.
 void launch_blend_backward(const BackwardIn& in, unsigned tiles, int tile_w, int tile_h, bool sparse, float* grad_pair,
                            cudaStream_t stream);
 // One view of one scene, everything the kernel reads about them in the frame's device tables: the

@@ -5,8 +5,9 @@
 // order, compiled without fast-math, so depth, rectangle and conic come out bit-identical to the
 // reference kernel built without --use_fast_math), then, fused into the same kernel:
 //   * writes the blend record (SplatRecord) and the tile rectangle of visible Gaussians;
-//   * writes every entry's depth key (the float bits of its depth; a sentinel if culled) -- the
-//     first LSD pass of the depth sort compacts the visible ones as it ranks them.
+//   * writes every entry's depth key (the float bits of its depth; a sentinel if culled);
+//   * counts each visible entry's tiles for the tile sort, or, for the LSD chain, its key's first digit
+//     (the chain's first pass compacts the visible entries as it ranks them).
 #include "common.cuh"
 #include "kernels.h"
 
@@ -104,8 +105,10 @@ struct Cov3 {
 
 // The rotation's products each occur in two sums, so which of a sum's two products the compiler rounds
 // before it fuses the other depends on the code around it. The choice is written out here, so that every
-// instantiation of the kernel gives a splat the same bits: kCrossXz (of the scene's layout) says whether
-// x z or w y is the rounded product of the two sums that hold both.
+// instantiation of the kernel for a layout gives a splat's covariance the same bits. The two layouts differ:
+// kCrossXz says whether x z (uploaded scenes) or w y (raw parameters) is the rounded product of the two sums
+// that hold both, as each had it when it was first compiled, so that neither's results moved. A render and
+// rasterize() of the same Gaussians can therefore differ by an ulp of the covariance.
 template <bool kCrossXz>
 __device__ __forceinline__ void covariance(const float4 sg, const float4 q, float splat_scale, Cov3& o) {
     const float w = q.x, x = q.y, y = q.z, z = q.w;
@@ -320,7 +323,7 @@ __device__ __forceinline__ bool project_entry(const Src& src, int64_t i, const f
     }
     rect16[e] = rect;
     // The depth key (the depth's bits less kDepthKeyBase: visible depths are >= 0.2, so the sign
-    // bit of kCulledKey never collides). The first depth pass compacts the visible entries.
+    // bit of kCulledKey never collides).
     const unsigned key = __float_as_uint(p.depth) - kDepthKeyBase;
     depth_key[e] = key;
     if (counts.counts) count_key(counts, count_blocks, e, key);
@@ -384,7 +387,7 @@ __device__ __forceinline__ void count_tiles(const TileCounts& tc, unsigned area,
 // where a warp's own 32 Gaussians have 14 visible on average. Outputs are indexed by entry, so the queue
 // order does not matter.
 //
-// Latency-bound (52% issue-active), held to 64 registers for eight CTAs of 128 threads per SM. Measured
+// Latency-bound (48% issue-active at 740k, 58% at 2.2M), held to 64 registers for eight CTAs of 128 threads per SM. Measured
 // at 2.2M / 1920x1080 (frame): 447 us with per-warp queues only, 430 us with the last items shared out
 // over 256 threads, 407 us with two Gaussians per thread (more of the warps have items to project),
 // 402 us with 128 threads (shorter waits for the CTA's slowest warp); at 740k / 1280x720: 198, 195, 195,

@@ -1,7 +1,7 @@
 // Steps 2-4 of the rasterizer: the stable (tile, depth, index) ordering of all splat-tile pairs.
-// The LSD chain: frames below kTileSortEntries entries (larger ones are sorted per tile, sort_tiles.cu),
-// frames of more than kTileSortTiles tiles and the sort of a given projection. Figures of larger frames
-// below were measured when this chain sorted them.
+// The LSD chain: frames below kTileSortEntries entries, frames of many visible entries per tile or of more than
+// kTileSortTiles tiles, and the sort of a given projection (the others are sorted per tile, sort_tiles.cu).
+// Figures of frames that the tile sort takes now were measured when this chain sorted them.
 //
 // The reference duplicates one 64-bit key (tile << 32 | depth bits) per pair in Gaussian-index order
 // and radix-sorts all of them over bits [0, 32 + bits(tiles)) (gpu_render.cu:148-161, 324-345).

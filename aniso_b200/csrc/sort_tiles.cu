@@ -1,5 +1,5 @@
 // The tile sort: the (tile, depth, index) order of all splat-tile pairs made per tile, for frames of
-// at least kTileSortEntries entries. Where the LSD chain (sort.cu) sorts the visible entries by depth
+// at least kTileSortEntries entries that do not crowd on few tiles (Plan::by_tile). Where the LSD chain (sort.cu) sorts the visible entries by depth
 // over the whole frame and then distributes them, here the pairs are distributed first and each
 // tile's list is sorted by itself, in shared memory:
 //   1. the preprocess cuts each visible entry's rectangle to the tiles its pixel bounds reach and counts
@@ -8,8 +8,8 @@
 //   3. tile_scatter appends every pair (depth key, entry) to its tile's list, in any order;
 //   4. tile_sort sorts each list by (depth key, entry) -- no two pairs of a tile are equal, so the order
 //      is unique and does not depend on the order of arrival: it is the reference's order. Lists of
-//      more than kTileChunk pairs are sorted in chunks, and tile_merge ranks each chunk's pairs among
-//      the other chunks of its list.
+//      more than kTileChunk pairs are sorted in chunks, and tile_merge merges each chunk with the other
+//      chunks of its list for its pairs' places.
 // Four short kernels (five for scenes of more Gaussians than a group of chunks holds, one more for
 // more tiles than one scan CTA adds up) where the chain has thirteen to eighteen, each latency-bound at a
 // few microseconds, and every pair is written twice instead of three to five times. Measured, frame

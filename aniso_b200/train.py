@@ -18,8 +18,8 @@
   `reset_every` steps clamp the opacities to twice the pruning threshold. New entries start with
   zero Adam moments, as gsplat's operations leave them.
 
-PyTorch holds the tensors and does the bookkeeping (concatenation, masks, the SSIM convolution); the
-rendering, the adjoint and the optimizer update are this library's kernels.
+PyTorch holds the tensors and does the bookkeeping (concatenation, masks); the rendering, the loss and its
+gradient, the adjoint and the optimizer update are this library's kernels.
 """
 from __future__ import annotations
 

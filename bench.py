@@ -45,9 +45,10 @@ N_GAUSS = 740_000
 # The reference's published GPU forward on its 0.74M-Gaussian *train* scene at 1280 wide:
 # 2.3 ms/frame on an RTX 5090 (README.md:28) = 741,883 / 2.3 ms.
 PUBLISHED_GAUSSIANS_PER_S = 741_883 / 2.3e-3
-# dram__bytes_read.sum + dram__bytes_write.sum of one blend launch on a ring view, from one ncu
-# capture of the bench command (the ncu summary of the blend kernel on this workload).
-BLEND_TRAFFIC_BYTES = 36_046_848
+# One blend launch on ring view 0, from an ncu capture (profiles/kernels_of_the_cases.md): DRAM bytes and
+# warp instructions (smsp__inst_executed.sum).
+BLEND_TRAFFIC_BYTES = 34_940_000
+BLEND_WARP_INSTRUCTIONS = 79_557_323
 
 
 def measured_peaks():
@@ -663,10 +664,12 @@ def main():
         # wait at the closing barrier, whose timeout minutes of rank-0-only work would exceed.
         base, acc = cpu_baseline_leg(gauss, sh, cams, images) if world == 1 else (None, None)
         ex2_peak, fma_peak = measured_compute_peaks()
-        # Algorithmic blend work: P * 256 pixel-splat evaluations per view (the upper bound; early
-        # termination counts as speed-up), one MUFU ex2 each.
-        evals = pairs_per_step / V * 256
-        evals_per_s = evals / (blend_ms / 1000.0)
+        # The blend is bound by instruction issue: its warp instructions against four a cycle and SM at the
+        # clock seen under load.
+        clocks = sampler.summary()
+        sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+        issue_peak = 4.0 * sms * 1e6 * (clocks.get("sm_mhz") or 0.0)
+        issued_per_s = BLEND_WARP_INSTRUCTIONS / (blend_ms / 1000.0)
         extra = {}
         if not args.no_extra and world == 1:
             extra["batched"] = batched_leg(torch, max(3, min(args.steps, 10)))
@@ -688,17 +691,15 @@ def main():
                        "vs_baseline_source": "reference README.md:28: 2.3 ms/frame, 0.74M train scene, RTX 5090"},
             "stages_ms_per_frame": {k: prof[k] / frames for k in ("project_ms", "sort_ms", "blend_ms")},
             "pairs_per_frame": pairs_per_step / V,
-            # The dominant kernel's roofline follows its bound: the blend issues one MUFU ex2 per
-            # pixel-splat evaluation (no stage is a dense contraction, and the blend reads far less
-            # than HBM could deliver), so its roofline is P*256 evaluations against the ex2 rate
-            # measured on this GPU; its HBM figure rides along.
-            "roofline": {"kernel": "blend", "bound": "mufu_ex2", "achieved": evals_per_s, "peak": ex2_peak,
-                         "unit": "ex2/s", "frac": (evals_per_s / ex2_peak) if ex2_peak else None,
-                         "peak_source": "measured on this GPU by the library's ex2 throughput probe "
-                                        "(libaniso_b200_peaks.so); MEASURED_PEAKS.json has no MUFU figure",
+            # The dominant kernel's roofline follows its bound, which is instruction issue (no stage is a
+            # dense contraction, the blend reads far less than HBM could deliver, and its exponentials take a
+            # fifth of the measured ex2 rate); its HBM figure rides along.
+            "roofline": {"kernel": "blend", "bound": "issue", "achieved": issued_per_s, "peak": issue_peak,
+                         "unit": "warp instructions/s", "frac": (issued_per_s / issue_peak) if issue_peak else None,
+                         "peak_source": "4 per cycle and SM at the SM clock sampled in the timed region",
                          "traffic": BLEND_TRAFFIC_BYTES,
-                         "work": "P*256 pixel-splat evaluations per view (the tile-area upper bound), one ex2 each",
-                         "fp32_fma_peak": fma_peak,
+                         "work": "warp instructions of the blend on ring view 0, counted by ncu",
+                         "ex2_peak": ex2_peak, "fp32_fma_peak": fma_peak,
                          "hbm": {"achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                                  "peak_source": peak_kind, "bytes": "P*40 + W*H*3 per launch"}},
             "stage_rooflines": stage_rooflines(prof, frames, counts, pairs_per_step / V, W, H, peak, peak_kind),
@@ -710,7 +711,7 @@ def main():
             "gpu_launches": launches_per_step * args.steps,
             "kernels_per_frame": launches_per_step / V,
             "timed_images_match_host_api": same,
-            "clocks": sampler.summary(),
+            "clocks": clocks,
         }
         line.update(extra)
         print(json.dumps(line), flush=True)

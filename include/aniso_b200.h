@@ -152,10 +152,12 @@ typedef struct aniso_b200_batch_options {
     float splat_scale;   /* as aniso_b200_options */
     int32_t tile_w;      /* tile shape: 8x8, 16x16 (the reference's, and the default for 0) or 16x32; */
     int32_t tile_h;      /*   the image is the same for every shape */
-    int32_t blend_batch; /* splats staged per blend round: < 256 the smaller, >= 256 the larger set */
+    int32_t blend_batch; /* splats staged per blend round: 128, or 256 from 256 on; no choice in 16x32
+                          * tiles (256) and in frames of under 32 Gaussians x views per tile (their own) */
     int32_t use_graph;   /* 1: record the launch sequence once as a CUDA graph and replay it */
-    int32_t radix_bits;  /* widest digit of the sort's tile passes: 8 (the default for 0) or 9, which
-                          * takes 9-bit digits where they save a pass (depth passes are always 8-bit) */
+    int32_t radix_bits;  /* widest digit of the tile passes where the sort is a chain of radix passes (under
+                          * 8192 Gaussians x views, or crowded on few tiles): 8 (the default for 0) or 9,
+                          * which takes 9-bit digits where they save a pass. Without effect elsewhere. */
 } aniso_b200_batch_options;
 
 /* A batch of n_views views; view k shows scene scenes[view_scene[k]]. The views of one scene must
